@@ -3,13 +3,17 @@
 // This is the true 32-bit matrix product of the engine (inputs, products and sums are
 // float; no tensor-core mode), and the plain twin that the tensor-core product is checked
 // against. Each output element is one fixed-order sum over K, whatever M is, so a row's
-// result does not depend on what else is in the batch. The reference runs these products
+// result does not depend on what else is in the batch: four chains over a quarter of K each, added
+// as (p0 + p1) + (p2 + p3) (gemm_f32.cuh; one chain over all of K leaves few threads to a decoding
+// row, and its rounding errors are twice as large). Float operands that can be read 16 bytes at a
+// time go to gemm_f32.cu, which forms the same sums. The reference runs these products
 // through nn.Linear (app/architectures/qwen_layers.py:50-53,
 // app/architectures/starcoder2_layers.py:19-23).
 //
 // Epilogue modes: 0 out(T) = v; 1 out(T) = gelu_tanh(v); 2 out(f32) = residual + v;
 // 3 out(f32) = v; 4 out(T) = max(v, 0)^2, where v = acc + bias.
 #include "common.cuh"
+#include "gemm_f32.cuh"
 
 namespace {
 
@@ -33,11 +37,12 @@ gemm_simt_kernel(const TIn* __restrict__ A, const TIn* __restrict__ W,
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int tx = tid % (BN / TN), ty = tid / (BN / TN);
 
-    float acc[TM][TN];
+    float acc[TM][TN], first[TM][TN], pair[TM][TN];      // the piece in hand; p0 + p1; p0 or p2
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < TN; ++j) acc[i][j] = first[i][j] = pair[i][j] = 0.f;
+    const int piece = f32_piece(K);
 
     // each thread stages 4 elements of A and 4 of W per k-tile: row = tid / 4, 4 k's at (tid % 4) * 4
     const int lrow = tid >> 2, lk = (tid & 3) << 2;
@@ -63,7 +68,23 @@ gemm_simt_kernel(const TIn* __restrict__ A, const TIn* __restrict__ W,
                 for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
         }
         __syncthreads();
+        if ((k0 + BK) % piece == 0 && k0 + BK < K) {         // a piece ends (its length is a multiple of BK)
+            const bool second = (k0 + BK) / piece == 2;
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    if (second) first[i][j] = pair[i][j] + acc[i][j];
+                    pair[i][j] = second ? 0.f : acc[i][j];
+                    acc[i][j] = 0.f;
+                }
+        }
     }
+    // the last piece that has any k: p0 or p2 stands alone, p1 or p3 joins the one before it
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = first[i][j] + (pair[i][j] + acc[i][j]);
 
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
@@ -98,6 +119,8 @@ extern "C" int mx_gemm_simt(const void* A, const void* W, int in_dtype, const fl
                   in_dtype, expected_out, out_dtype);
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) MX_REFUSE("gemm: M = %d is beyond this kernel's grid", M);
+    if (in_dtype == MX_DTYPE_F32 && mx_gemm_f32_takes((const float*)A, lda, (const float*)W, ldw, N, K))
+        return mx_gemm_f32((const float*)A, lda, (const float*)W, ldw, bias, residual, (float*)out, ldo, M, N, K, mode, stream);
 #define MX_GEMM(TI, TO) \
     gemm_simt_kernel<TI, TO><<<grid, THREADS, 0, stream>>>((const TI*)A, (const TI*)W, bias, residual, (TO*)out, M, N, K, lda, ldw, ldo, mode, 0, 0, 0, 0)
     if (in_dtype == MX_DTYPE_F32 && out_dtype == MX_DTYPE_F32) MX_GEMM(float, float);
