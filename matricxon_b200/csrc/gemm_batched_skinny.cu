@@ -1,10 +1,18 @@
 // Many small independent products with at most 16 rows each (the per-head and per-block products of a
 // decode step): out[m][b][n] = sum_k A[m][b][k] * W[b][n][k], bfloat16 in, float accumulation.
 //
-// One warp per output column (b, n): the weight row is read once with 16-byte loads (lane l takes the
+// K a multiple of 32: a block of four warps forms 16 columns of a member on the tensor cores (mma.sync, the columns'
+// weight rows as its 16 rows, the rows of A as its 8 columns, one or two of them). Warp w takes the blocks of 32 k
+// numbered w, w + 4, ..., every thread 16 contiguous bytes of two weight rows and of a row of A a block, the
+// contraction permuted the same way on both sides, and the warps' sums are added in a fixed order, so a row's
+// result does not depend on the other rows. The products are a few microseconds of launches and latencies (16 heads of
+// 512 x 128 are 2 MB): the first weights set out before the wait on the kernel that makes A.
+// Other K: one warp per output column (b, n): the weight row is read once with 16-byte loads (lane l takes the
 // elements 8l .. 8l+7 of every block of 256), every row of A against it, and the lanes' partial sums are
-// added by shuffles in a fixed order, so a row's result does not depend on the other rows. The operands
-// of the batch members may interleave (heads side by side in a row): rows are lda / ldo apart, members
+// added by shuffles in a fixed order. Sixteen requests decoding with four latent
+// attentions and two gated recurrences (ten of these products) took 801 us a step that way, on the tensor cores 691: a
+// multiply-add a lane and element, half of the lanes idle at K = 128, and eighty shuffles a column were 17 us a product.
+// The operands of the batch members may interleave (heads side by side in a row): rows are lda / ldo apart, members
 // a_batch / w_batch / o_batch apart. Takes part in chained launches. K must be a multiple of 8 and every row 16-byte aligned.
 #include "common.cuh"
 
@@ -58,6 +66,99 @@ batched_skinny_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* 
     }
 }
 
+__device__ __forceinline__ void bs_mma(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
+                                       unsigned b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+constexpr int BM_WARPS = 4, BM_AHEAD = 4;      // BM_AHEAD: blocks of 32 k whose weights a thread holds at a time
+
+template <typename TOut, int MB>
+__global__ void __launch_bounds__(BM_WARPS * 32)
+batched_mma_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ W, TOut* __restrict__ out, int M,
+                   int N, int K, int lda, int ldw, int ldo, int tiles, long long a_batch, long long w_batch,
+                   long long o_batch) {
+    __shared__ float sums[BM_WARPS][16][8 * MB];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int b = blockIdx.x / tiles, n0 = (blockIdx.x - b * tiles) * 16;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    const __nv_bfloat16* w_row[2];
+    bool w_in[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        w_in[i] = n0 + g + 8 * i < N;
+        w_row[i] = W + (size_t)b * w_batch + (size_t)min(n0 + g + 8 * i, N - 1) * ldw + 8 * t;
+    }
+    const int blocks = K / 32;
+    uint4 wf[BM_AHEAD][2];
+    auto weights = [&](int kb0) {
+#pragma unroll
+        for (int u = 0; u < BM_AHEAD; ++u)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int kb = kb0 + u * BM_WARPS;
+                wf[u][i] = kb < blocks && w_in[i] ? *reinterpret_cast<const uint4*>(w_row[i] + 32 * kb) : zero;
+            }
+    };
+    weights(warp);
+    pdl_trigger();
+    pdl_wait();
+    const __nv_bfloat16* a_row[MB];
+    bool a_in[MB];
+#pragma unroll
+    for (int mb = 0; mb < MB; ++mb) {
+        a_in[mb] = 8 * mb + g < M;
+        a_row[mb] = after_wait(A) + (size_t)b * a_batch + (size_t)min(8 * mb + g, M - 1) * lda + 8 * t;
+    }
+    float acc[MB][4];
+#pragma unroll
+    for (int mb = 0; mb < MB; ++mb) acc[mb][0] = acc[mb][1] = acc[mb][2] = acc[mb][3] = 0.f;
+    for (int kb0 = warp; kb0 < blocks; kb0 += BM_AHEAD * BM_WARPS) {
+        if (kb0 != warp) weights(kb0);
+        uint4 af[BM_AHEAD][MB];
+#pragma unroll
+        for (int u = 0; u < BM_AHEAD; ++u)
+#pragma unroll
+            for (int mb = 0; mb < MB; ++mb) {
+                const int kb = kb0 + u * BM_WARPS;
+                af[u][mb] = kb < blocks && a_in[mb] ? *reinterpret_cast<const uint4*>(a_row[mb] + 32 * kb) : zero;
+            }
+#pragma unroll
+        for (int u = 0; u < BM_AHEAD; ++u)
+#pragma unroll
+            for (int mb = 0; mb < MB; ++mb) {
+                bs_mma(acc[mb], wf[u][0].x, wf[u][1].x, wf[u][0].y, wf[u][1].y, af[u][mb].x, af[u][mb].y);
+                bs_mma(acc[mb], wf[u][0].z, wf[u][1].z, wf[u][0].w, wf[u][1].w, af[u][mb].z, af[u][mb].w);
+            }
+    }
+    // this thread holds columns g and g + 8 for rows 8 mb + 2t, + 1
+#pragma unroll
+    for (int mb = 0; mb < MB; ++mb)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sums[warp][g + 8 * (e >> 1)][8 * mb + 2 * t + (e & 1)] = acc[mb][e];
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < 16 * 8 * MB; idx += BM_WARPS * 32) {
+        const int f = idx % 16, m = idx / 16;
+        if (n0 + f >= N || m >= M) continue;
+        float v = sums[0][f][m];
+#pragma unroll
+        for (int w = 1; w < BM_WARPS; ++w) v += sums[w][f][m];
+        out[(size_t)m * ldo + (size_t)b * o_batch + n0 + f] = from_float<TOut>(v);
+    }
+}
+
+template <typename TOut>
+cudaError_t launch_mma(const void* A, const void* W, void* out, int M, int N, int K, int lda, int ldw, int ldo, int batch,
+                       long long a_batch, long long w_batch, long long o_batch, cudaStream_t stream) {
+    const int tiles = (N + 15) / 16;
+    return mx_launch_chained(M <= 8 ? batched_mma_kernel<TOut, 1> : batched_mma_kernel<TOut, 2>,
+                             dim3((unsigned)(tiles * (long long)batch)), dim3(BM_WARPS * 32), 0, stream,
+                             (const __nv_bfloat16*)A, (const __nv_bfloat16*)W, (TOut*)out, M, N, K, lda, ldw, ldo, tiles,
+                             a_batch, w_batch, o_batch);
+}
+
 }  // namespace
 
 extern "C" int mx_gemm_batched_skinny(const void* A, const void* W, void* out, int out_dtype, int M, int N, int K,
@@ -67,6 +168,13 @@ extern "C" int mx_gemm_batched_skinny(const void* A, const void* W, void* out, i
     if (M > BS_ROWS) MX_REFUSE("batched skinny product: %d rows exceed %d", M, BS_ROWS);
     if (K <= 0 || K % 8 || lda % 8 || ldw % 8 || a_batch % 8 || w_batch % 8)
         MX_REFUSE("batched skinny product: K = %d and the strides must be multiples of 8", K);
+    if (K % 32 == 0) {
+        const cudaError_t e = out_dtype == MX_DTYPE_F32
+                                  ? launch_mma<float>(A, W, out, M, N, K, lda, ldw, ldo, batch, a_batch, w_batch, o_batch, stream)
+                                  : launch_mma<__nv_bfloat16>(A, W, out, M, N, K, lda, ldw, ldo, batch, a_batch, w_batch, o_batch, stream);
+        if (e != cudaSuccess) mx_set_error("batched skinny product: launch failed: %s", cudaGetErrorString(e));
+        return (int)e;
+    }
     const long long columns = (long long)batch * N;
     const unsigned blocks = (unsigned)((columns + BS_WARPS - 1) / BS_WARPS);
     if (out_dtype == MX_DTYPE_F32)
