@@ -15,23 +15,27 @@
 //                      head dim) and per chunk the keys, warp 10 the values: TMA boxes straight out
 //                      of the paged cache, one page per lane, page numbers from the block table
 //                      (read once per tile into shared memory), two stages each. A key stage is
-//                      free as soon as its Q K^T has run, a value stage when its P V has;
-//   warp 9 (one lane)  issues S = Q K^T (tcgen05.mma, operands in swizzled shared memory,
-//                      accumulator in tensor memory, three S buffers so that the scores of the
+//                      free as soon as its Q K^T has run, a value stage when its P V has. The queries
+//                      and the first keys set out before the block has set itself up;
+//   warp 9             issues S = Q K^T (tcgen05.mma, operands in swizzled shared memory,
+//                      accumulator in tensor memory, two S buffers so that the scores of the
 //                      next chunk exist before the softmax of this one ends) and O += P V (P read
-//                      from tensor memory, V^T pages as the K-major B operand, O in tensor memory);
-//   warps 0-7          softmax: two threads per row (warps w and w + 4 reach the same quarter of
-//                      tensor memory), each with 64 of the chunk's 128 keys. A thread reads its
-//                      scores from tensor memory (tcgen05.ld), masks the chunks that cross an edge,
-//                      exchanges its maximum with its partner through shared memory, keeps a running
-//                      reference maximum that only moves when the new maximum exceeds it by 2^8
-//                      (then O is rescaled in tensor memory), writes P as bfloat16 over the first
-//                      64 columns of the same score buffer (tcgen05.st), and at the end
-//                      normalises its 64 columns of O and stores them. (One thread per row took
-//                      82 us for the 2,048-token portion of the 3B sizes, two take 75: a scheduler
-//                      with two softmax warps runs one's tensor-memory loads under the other's
-//                      exponentials. The chunk's 16,384 exponentials alone are 1,024 cycles of the
-//                      SM's special-function units, as long as its MMAs.)
+//                      from tensor memory, V^T pages as the K-major B operand), an O for each half of
+//                      a chunk's keys;
+//   warps 0-7          softmax: two threads per row, each with 64 of the chunk's 128 keys: warps 0-3
+//                      the first 64, warps 4-7 the others, as two independent online softmaxes with a
+//                      reference maximum, a sum and an O of their own that are joined at the end. A
+//                      thread reads its scores from tensor memory (tcgen05.ld), masks the chunks that
+//                      cross an edge, keeps a running reference maximum that only moves when the new
+//                      maximum exceeds it by 2^8 (then its O is rescaled in tensor memory), writes P as
+//                      bfloat16 over its own columns of the score buffer (tcgen05.st), and at the end
+//                      joins and normalises 64 columns of the two O and stores them.
+// Measured at the 3B sizes (24 query heads on 2 KV heads): 2,048 tokens 58 us (447 TFLOP/s; one softmax
+// in step over all 128 keys, tiles in the order of their tokens: 76), 512 tokens after 512: 18 us (27), 512
+// after 4,000: 48 us (65). A chunk takes 2,050 cycles; its MMAs alone would take 1,024, its 16,384
+// exponentials on the special-function units as many. What bounds it is latency: two softmax warps a scheduler
+// issue a third of the time, either unit is busy a third of the time. Handing the exponentials from half to half,
+// Q K^T of each half on its own, and exponentials in batches of sixteen each measured 2 to 5 % slower.
 // Keys beyond the newest one of the tile are not data yet: their scores are masked by selection and
 // their value columns are zeroed in shared memory before the last P V (0 x NaN must not happen).
 // Every mbarrier wait is bounded: a wait that runs out sets MX_STATUS_WAIT_TIMEOUT and the role
@@ -47,27 +51,25 @@ constexpr int AT_ROWS = 128;
 constexpr int AT_KEYS = 128;
 constexpr int AT_HD = 128;
 constexpr int AT_STAGES = 2;
-constexpr int AT_SOFTMAX_WARPS = 8;                    // two per quarter of tensor memory: each takes half of a row's keys
+constexpr int AT_SOFTMAX_WARPS = 8;                    // two sets of four: each takes half of every chunk's keys
 constexpr int AT_SOFTMAX_THREADS = AT_SOFTMAX_WARPS * 32;
 constexpr int AT_KEY_WARP = 8, AT_MMA_WARP = 9, AT_VALUE_WARP = 10;
 constexpr int AT_THREADS = 352;                       // warps 0-7 softmax, 8 keys, 9 MMA, 10 values
 constexpr unsigned AT_SPIN = 1u << 18;
 constexpr int AT_TILE = AT_ROWS * 64 * 2;            // bytes of a [128][64] bfloat16 half tile
-constexpr int AT_SBUF = 3;                            // score buffers in tensor memory: 3 x 128 columns, then O
+constexpr int AT_SBUF = 2;                            // score buffers in tensor memory: 2 x 128 columns, then two O
 constexpr int AT_TABLE = 1024;                        // block-table entries of a tile kept in shared memory
 constexpr float AT_JUMP = 8.f;                        // log2 of the growth the reference maximum tolerates
 
 struct AtShared {
     unsigned long long q_full;
     unsigned long long k_full[AT_STAGES], v_full[AT_STAGES];
-    // three S buffers (P of a chunk overwrites its S): Q K^T runs two chunks ahead of P V, and a softmax
-    // warp may be up to two chunks ahead of another, so every barrier of a chunk is per buffer
-    unsigned long long s_full[AT_SBUF], p_full[AT_SBUF];
-    // completion of the P V of even and of odd chunks: the value producer, about to refill the stage of
-    // chunk j - 2, and the softmax threads wait on it; with two barriers neither can fall two phases behind
-    unsigned long long pv_done[2];
+    // two S buffers (P of a chunk overwrites its S): the scores of chunk j + 1 are issued before P V of chunk j.
+    // P and the completion of P V are per half of the keys; all are counted per buffer, so that no wait can be
+    // two phases behind.
+    unsigned long long s_full[AT_SBUF], p_full[2][AT_SBUF], pv_done[2][2];
     unsigned tmem_base;
-    int abort;                   // a softmax thread's wait ran out: all of them leave at the next exchange
+    int abort;                   // a softmax thread's wait ran out: nothing is stored
 };
 
 struct AtParams {
@@ -81,7 +83,7 @@ struct AtParams {
     int n_splits;                // blockIdx.z takes every n_splits-th share of a tile's chunks of keys
     int* status;
     long long n_pages;
-    int out_stride, bt_stride, n_heads, n_kv_heads, group, tokens_per_tile, page_size, page_shift, window;
+    int n_tiles, out_stride, bt_stride, n_heads, n_kv_heads, group, tokens_per_tile, page_size, page_shift, window;
     int keep;                    // under a window: keys at positions below this are seen at any distance
     float scale_log2;
     // capped scores: cap_log2 = cap * log2(e) > 0 turns score * scale into cap * tanh(score * scale / cap)
@@ -112,7 +114,7 @@ __device__ __forceinline__ bool at_try_wait(unsigned long long* bar, unsigned pa
         : "memory");
     return ok != 0;
 }
-// false: the wait ran out (status set); the caller leaves its loop
+// false: the wait ran out (status set; by a whole warp, by each of its lanes); the caller leaves its loop
 __device__ __forceinline__ bool at_wait(unsigned long long* bar, unsigned parity, int* status) {
     for (unsigned spin = 0; spin < AT_SPIN; ++spin)
         if (at_try_wait(bar, parity)) return true;
@@ -153,12 +155,15 @@ __device__ __forceinline__ unsigned at_idesc(int m, int n) {
     d |= (unsigned)(m >> 4) << 24;
     return d;
 }
+// The whole warp issues these (warp index uniform, one elected lane does): a lone lane's loop runs in divergent code,
+// where each operand is moved to a uniform register on its own, about 90 cycles an instruction (tcgen05_helpers.cuh).
 __device__ __forceinline__ void at_mma(unsigned tmem_acc, unsigned long long adesc, unsigned long long bdesc,
                                        unsigned idesc, bool accumulate) {
     asm volatile(
-        "{\n.reg .pred p;\n"
+        "{\n.reg .pred p, q;\n"
+        "elect.sync _|q, 0xffffffff;\n"
         "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_acc),
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_acc),
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"((unsigned)accumulate)
         : "memory");
 }
@@ -166,9 +171,10 @@ __device__ __forceinline__ void at_mma(unsigned tmem_acc, unsigned long long ade
 __device__ __forceinline__ void at_mma_ts(unsigned tmem_acc, unsigned tmem_a, unsigned long long bdesc, unsigned idesc,
                                           bool accumulate) {
     asm volatile(
-        "{\n.reg .pred p;\n"
+        "{\n.reg .pred p, q;\n"
+        "elect.sync _|q, 0xffffffff;\n"
         "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_acc),
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_acc),
         "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"((unsigned)accumulate)
         : "memory");
 }
@@ -184,8 +190,11 @@ __device__ __forceinline__ void tmem_store32_bits(unsigned taddr, const unsigned
         : "memory");
 }
 __device__ __forceinline__ void at_commit(unsigned long long* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar))
-                 : "memory");
+    asm volatile(
+        "{\n.reg .pred q;\n"
+        "elect.sync _|q, 0xffffffff;\n"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_u32(bar))
+        : "memory");
 }
 __device__ __forceinline__ void tmem_load32(unsigned taddr, float* v) {
     unsigned r[32];
@@ -240,9 +249,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     unsigned char* k_stage = q_tile + 2 * AT_TILE;                  // per stage: 2 halves of [128 keys][64]
     unsigned char* v_stage = k_stage + AT_STAGES * 2 * AT_TILE;     // per stage: pages of [128 dims][page_size]
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int seq = p.tiles[2 * blockIdx.x], tok0 = p.tiles[2 * blockIdx.x + 1];
-    const int kh = blockIdx.y;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    // a sequence's last tiles see the most keys: they start first, all heads of a tile side by side
+    const int tile = p.n_tiles - 1 - (int)(blockIdx.x / (unsigned)p.n_kv_heads);
+    const int kh = (int)(blockIdx.x % (unsigned)p.n_kv_heads);
+    const int seq = p.tiles[2 * tile], tok0 = p.tiles[2 * tile + 1];
     const int q_start = p.cu_q[seq];
     const int q_len = p.cu_q[seq + 1] - q_start;
     const int ctx = p.context_lens[seq];
@@ -275,30 +286,91 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     const int pages_per_chunk = AT_KEYS >> p.page_shift;
     const unsigned page_bytes = (unsigned)(p.page_size * AT_HD * 2);
 
-    if (tid == 0) {
-        at_mbar_init(&sh.q_full, 1);
-        for (int s = 0; s < AT_STAGES; ++s) {
-            at_mbar_init(&sh.k_full[s], 1);
-            at_mbar_init(&sh.v_full[s], 1);
+    const int* bt = p.block_tables + (size_t)seq * p.bt_stride;
+    auto logical_page = [&](int i) {              // the i-th page of this block's list of chunks
+        const int j = i / pages_per_chunk;
+        return ((chunk_of(j) * AT_KEYS) >> p.page_shift) + (i - j * pages_per_chunk);
+    };
+    // this tile's part of the block table, read once by each producer (entries beyond AT_TABLE stay in global memory)
+    auto read_table = [&](int* table) {
+        const int n_table = min(n_chunks * pages_per_chunk, AT_TABLE);
+        for (int i = lane; i < n_table; i += 32) {
+            const int lp = logical_page(i);
+            table[i] = lp < p.bt_stride ? bt[lp] : -1;
         }
-        for (int b = 0; b < AT_SBUF; ++b) {
-            at_mbar_init(&sh.s_full[b], 1);
-            at_mbar_init(&sh.p_full[b], AT_SOFTMAX_WARPS);
+        __syncwarp();
+    };
+    // the keys (or the values) of chunk j into stage j % AT_STAGES: lane pg brings page pg
+    auto bring = [&](int j, bool keys, const int* table) {
+        const int s = j % AT_STAGES;
+        unsigned long long* full = keys ? &sh.k_full[s] : &sh.v_full[s];
+        const int c0 = chunk_of(j) * AT_KEYS;
+        long long page = -1;
+        if (lane < pages_per_chunk) {
+            const int key0 = c0 + lane * p.page_size;
+            if (key0 <= hi_tile && (key0 + p.page_size - 1 >= lo_tile || key0 < p.keep)) {
+                const int i = j * pages_per_chunk + lane;
+                const int lp = logical_page(i);
+                page = i < AT_TABLE ? table[i] : (lp < p.bt_stride ? bt[lp] : -1);
+                if (page < 0 || page >= p.n_pages) {
+                    page = -1;
+                    if (keys) atomicOr(p.status, MX_STATUS_BAD_PAGE);
+                }
+            }
         }
-        at_mbar_init(&sh.pv_done[0], 1);
-        at_mbar_init(&sh.pv_done[1], 1);
-        sh.abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    // value stages start as zeros: a page that is never fetched must not hold NaN bit patterns
-    for (int i = tid; i < AT_STAGES * 2 * AT_TILE / 16; i += AT_THREADS)
-        reinterpret_cast<uint4*>(v_stage)[i] = make_uint4(0u, 0u, 0u, 0u);
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    if (warp == AT_MMA_WARP) {
+        const unsigned n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0));
+        if (lane == 0) at_expect_tx(full, n_valid * page_bytes);
+        __syncwarp();
+        if (page >= 0) {
+            const int block = (int)(page * 2 * p.n_kv_heads) + kh;
+            if (keys) {
+                unsigned char* ks = k_stage + (size_t)s * 2 * AT_TILE + (size_t)lane * p.page_size * 128;
+                tma_3d(ks, &k_map, 0, 0, block, full);
+                tma_3d(ks + AT_TILE, &k_map, 64, 0, block, full);
+            } else {
+                tma_3d(v_stage + (size_t)s * 2 * AT_TILE + (size_t)lane * page_bytes, &v_map, 0, 0,
+                       block + p.n_kv_heads, full);
+            }
+        }
+        __syncwarp();
+    };
+    // What the first scores wait for sets out at once, under the rest of the setup: the key producer makes the
+    // barriers itself and asks for the queries and the first keys before the block meets.
+    if (warp == AT_KEY_WARP) {
+        if (lane == 0) {
+            at_mbar_init(&sh.q_full, 1);
+            for (int s = 0; s < AT_STAGES; ++s) {
+                at_mbar_init(&sh.k_full[s], 1);
+                at_mbar_init(&sh.v_full[s], 1);
+            }
+            for (int b = 0; b < AT_SBUF; ++b) {
+                at_mbar_init(&sh.s_full[b], 1);
+                for (int half = 0; half < 2; ++half) at_mbar_init(&sh.p_full[half][b], AT_SOFTMAX_WARPS / 2);
+            }
+            for (int half = 0; half < 2; ++half)
+                for (int b = 0; b < 2; ++b) at_mbar_init(&sh.pv_done[half][b], 1);
+            sh.abort = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+            const unsigned q_bytes = (unsigned)(2 * 64 * p.group * p.tokens_per_tile * 2);   // boxes count in full
+            at_expect_tx(&sh.q_full, q_bytes);
+            tma_4d(q_tile, &q_map, 0, 0, kh, q_start + tok0, &sh.q_full);
+            tma_4d(q_tile + AT_TILE, &q_map, 64, 0, kh, q_start + tok0, &sh.q_full);
+        }
+        __syncwarp();
+        read_table(table_k);
+        bring(0, true, table_k);
+    } else if (warp == AT_MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&sh.tmem_base)),
                      "r"(512)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    } else if (warp == AT_VALUE_WARP) {
+        read_table(table_v);
+    } else {
+        // value stages start as zeros: a page that is never fetched must not hold NaN bit patterns
+        for (int i = tid; i < AT_STAGES * 2 * AT_TILE / 16; i += AT_SOFTMAX_THREADS)
+            reinterpret_cast<uint4*>(v_stage)[i] = make_uint4(0u, 0u, 0u, 0u);
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
@@ -307,189 +379,115 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     const unsigned tmem_o = tmem_base + AT_SBUF * 128;
 
     if (warp == AT_KEY_WARP || warp == AT_VALUE_WARP) {
-        // ---------------- producers: warp 4 brings the query tile and the keys, warp 6 the values, each
-        // at its own pace (a key stage is free once its Q K^T is done, a value stage once its P V is);
-        // lane pg owns page pg of every chunk
+        // ---------------- producers, each at its own pace: a stage held chunk j - 2, whose keys are free once that
+        // chunk's scores exist, whose values are once both of its P V have run (the second one's commit says so)
         const bool keys = warp == AT_KEY_WARP;
-        int* table = keys ? table_k : table_v;
-        const int* bt = p.block_tables + (size_t)seq * p.bt_stride;
-        if (keys && lane == 0) {
-            const unsigned q_bytes = (unsigned)(2 * 64 * p.group * p.tokens_per_tile * 2);   // boxes count in full
-            at_expect_tx(&sh.q_full, q_bytes);
-            tma_4d(q_tile, &q_map, 0, 0, kh, q_start + tok0, &sh.q_full);
-            tma_4d(q_tile + AT_TILE, &q_map, 64, 0, kh, q_start + tok0, &sh.q_full);
-        }
-        // this tile's part of the block table, read once (entries beyond AT_TABLE stay in global memory)
-        auto logical_page = [&](int i) {          // the i-th page of this block's list of chunks
-            const int j = i / pages_per_chunk;
-            return ((chunk_of(j) * AT_KEYS) >> p.page_shift) + (i - j * pages_per_chunk);
-        };
-        const int n_table = min(n_chunks * pages_per_chunk, AT_TABLE);
-        for (int i = lane; i < n_table; i += 32) {
-            const int lp = logical_page(i);
-            table[i] = lp < p.bt_stride ? bt[lp] : -1;
-        }
-        __syncwarp();
-        for (int j = 0; j < n_chunks; ++j) {
-            const int s = j % AT_STAGES;
-            unsigned long long* full = keys ? &sh.k_full[s] : &sh.v_full[s];
-            bool free_now = true;
-            if (lane == 0 && j >= AT_STAGES) {
-                // the stage held chunk j - 2: its keys are free once that chunk's scores exist, its values
-                // once that chunk's P V has run
+        for (int j = keys ? 1 : 0; j < n_chunks; ++j) {
+            if (j >= AT_STAGES) {
                 const int before = j - AT_STAGES;
-                free_now = keys ? at_wait(&sh.s_full[before % AT_SBUF], (unsigned)(before / AT_SBUF) & 1, p.status)
-                                : at_wait(&sh.pv_done[before & 1], (unsigned)(before >> 1) & 1, p.status);
+                const unsigned parity = (unsigned)(before >> 1) & 1;
+                if (!__all_sync(0xffffffffu, keys ? at_wait(&sh.s_full[before & 1], parity, p.status)
+                                                  : at_wait(&sh.pv_done[1][before & 1], parity, p.status))) break;
             }
-            if (!__shfl_sync(0xffffffffu, free_now, 0)) break;
-            const int c0 = chunk_of(j) * AT_KEYS;
-            long long page = -1;
-            if (lane < pages_per_chunk) {
-                const int key0 = c0 + lane * p.page_size;
-                if (key0 <= hi_tile && (key0 + p.page_size - 1 >= lo_tile || key0 < p.keep)) {
-                    const int i = j * pages_per_chunk + lane;
-                    const int lp = logical_page(i);
-                    page = i < AT_TABLE ? table[i] : (lp < p.bt_stride ? bt[lp] : -1);
-                    if (page < 0 || page >= p.n_pages) {
-                        page = -1;
-                        if (keys) atomicOr(p.status, MX_STATUS_BAD_PAGE);
-                    }
-                }
-            }
-            const unsigned n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0));
-            if (lane == 0) at_expect_tx(full, n_valid * page_bytes);
-            __syncwarp();
-            if (page >= 0) {
-                const int block = (int)(page * 2 * p.n_kv_heads) + kh;
-                if (keys) {
-                    unsigned char* ks = k_stage + (size_t)s * 2 * AT_TILE + (size_t)lane * p.page_size * 128;
-                    tma_3d(ks, &k_map, 0, 0, block, full);
-                    tma_3d(ks + AT_TILE, &k_map, 64, 0, block, full);
-                } else {
-                    tma_3d(v_stage + (size_t)s * 2 * AT_TILE + (size_t)lane * page_bytes, &v_map, 0, 0,
-                           block + p.n_kv_heads, full);
-                }
-            }
+            bring(j, keys, keys ? table_k : table_v);
         }
     } else if (warp == AT_MMA_WARP) {
-        // ---------------- MMA issuer. One thread; everything it can know before the loop is computed
-        // there, and a chunk costs it two commits: tcgen05.mma of one thread run in issue order, so the
-        // Q K^T that overwrites a score buffer needs no barrier against the P V that read P from it.
-        if (lane == 0) {
-            const unsigned idesc = at_idesc(AT_ROWS, AT_KEYS);
-            const unsigned v_layout = p.page_size == 16 ? 6u : 4u;       // 32- or 64-byte swizzle
-            const unsigned v_sbo = (unsigned)(8 * p.page_size * 2);       // eight rows of one page tile
-            const int steps_per_page = p.page_size / 16;
-            unsigned long long q_desc[2], k_desc[AT_STAGES][2], v_desc[AT_STAGES];
-            unsigned v_step[AT_KEYS / 16];                                 // where the 16 keys of step kk start
+        // ---------------- MMA issuer: the whole warp walks the loop, one elected lane issues. tcgen05.mma of one
+        // thread run in issue order, so the Q K^T that overwrites a score buffer needs no barrier against the
+        // P V that read P from it.
+        const unsigned idesc = at_idesc(AT_ROWS, AT_KEYS);
+        const unsigned v_layout = p.page_size == 16 ? 6u : 4u;       // 32- or 64-byte swizzle
+        const unsigned v_sbo = (unsigned)(8 * p.page_size * 2);       // eight rows of one page tile
+        const int steps_per_page = p.page_size / 16;
+        const unsigned long long q_desc = at_desc(q_tile, 1024, 2), k_desc = at_desc(k_stage, 1024, 2);
+        const unsigned long long v_desc = at_desc(v_stage, v_sbo, v_layout);
+        unsigned v_step[AT_KEYS / 16];                                 // where the 16 keys of step kk start
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                q_desc[half] = at_desc(q_tile + half * AT_TILE, 1024, 2);
+        for (int kk = 0; kk < AT_KEYS / 16; ++kk) {
+            const int pg = kk / steps_per_page, within = kk - pg * steps_per_page;
+            v_step[kk] = (unsigned)((pg * page_bytes) >> 4) + 2u * within;
+        }
+        auto issue_qk = [&](int j) -> bool {
+            const int st = j % AT_STAGES;
+            if (!__all_sync(0xffffffffu, at_wait(&sh.k_full[st], (unsigned)(j / AT_STAGES) & 1, p.status))) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const unsigned acc = tmem_base + (unsigned)(j % AT_SBUF) * 128;
+            const unsigned long long kd = k_desc + (unsigned long long)st * (2 * AT_TILE >> 4);
 #pragma unroll
-                for (int st = 0; st < AT_STAGES; ++st)
-                    k_desc[st][half] = at_desc(k_stage + (size_t)st * 2 * AT_TILE + half * AT_TILE, 1024, 2);
-            }
+            for (int half = 0; half < 2; ++half)                       // of the head dim
 #pragma unroll
-            for (int st = 0; st < AT_STAGES; ++st) v_desc[st] = at_desc(v_stage + (size_t)st * 2 * AT_TILE, v_sbo, v_layout);
+                for (int k = 0; k < 4; ++k)
+                    at_mma(acc, q_desc + half * (AT_TILE >> 4) + 2 * k, kd + half * (AT_TILE >> 4) + 2 * k, idesc, (half | k) != 0);
+            at_commit(&sh.s_full[j % AT_SBUF]);
+            return true;
+        };
+        bool alive = __all_sync(0xffffffffu, at_wait(&sh.q_full, 0, p.status));
+        if (alive) alive = issue_qk(0);
+        for (int j = 0; j < n_chunks && alive; ++j) {
+            // the scores of the next chunk, before this chunk's P V
+            if (j + 1 < n_chunks && !issue_qk(j + 1)) break;
+            const unsigned p_addr = tmem_base + (unsigned)(j % AT_SBUF) * 128;
+            const unsigned long long vd = v_desc + (unsigned long long)(j % AT_STAGES) * (2 * AT_TILE >> 4);
+            alive = __all_sync(0xffffffffu, at_wait(&sh.v_full[j % AT_STAGES], (unsigned)(j / AT_STAGES) & 1, p.status));
 #pragma unroll
-            for (int kk = 0; kk < AT_KEYS / 16; ++kk) {
-                const int pg = kk / steps_per_page, within = kk - pg * steps_per_page;
-                v_step[kk] = (unsigned)((pg * page_bytes) >> 4) + 2u * within;
-            }
-            bool alive = at_wait(&sh.q_full, 0, p.status);
-            // state of the chunk whose scores are issued next (qk_*) and of the chunk whose P V is next (pv_*)
-            int qk_stage = 0, qk_buf = 0;
-            unsigned qk_stage_parity = 0;
-            auto issue_qk = [&]() -> bool {
-                if (!at_wait(&sh.k_full[qk_stage], qk_stage_parity, p.status)) return false;
+            for (int half = 0; half < 2; ++half) {                     // of the keys
+                if (alive) alive = __all_sync(0xffffffffu, at_wait(&sh.p_full[half][j % AT_SBUF], (unsigned)(j / AT_SBUF) & 1, p.status));
+                if (!alive) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const unsigned acc = tmem_base + (unsigned)qk_buf * 128;
 #pragma unroll
-                for (int half = 0; half < 2; ++half)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        at_mma(acc, q_desc[half] + 2 * k, k_desc[qk_stage][half] + 2 * k, idesc, (half | k) != 0);
-                at_commit(&sh.s_full[qk_buf]);
-                if (++qk_stage == AT_STAGES) {
-                    qk_stage = 0;
-                    qk_stage_parity ^= 1u;
-                }
-                if (++qk_buf == AT_SBUF) qk_buf = 0;
-                return true;
-            };
-            if (alive) alive = issue_qk();
-            int pv_stage = 0, pv_buf = 0;
-            unsigned pv_stage_parity = 0, pv_buf_parity = 0;
-            for (int j = 0; j < n_chunks && alive; ++j) {
-                if (j + 1 < n_chunks) {           // the scores of the next chunk, before this chunk's P V
-                    alive = issue_qk();
-                    if (!alive) break;
-                }
-                if (!at_wait(&sh.p_full[pv_buf], pv_buf_parity, p.status)) break;
-                if (!at_wait(&sh.v_full[pv_stage], pv_stage_parity, p.status)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const unsigned p_addr = tmem_base + (unsigned)pv_buf * 128;
-#pragma unroll
-                for (int kk = 0; kk < AT_KEYS / 16; ++kk)             // 16 keys per MMA: 8 columns of P
-                    at_mma_ts(tmem_o, p_addr + 8 * kk, v_desc[pv_stage] + v_step[kk], idesc, (j | kk) != 0);
-                at_commit(&sh.pv_done[j & 1]);
-                if (++pv_stage == AT_STAGES) {
-                    pv_stage = 0;
-                    pv_stage_parity ^= 1u;
-                }
-                if (++pv_buf == AT_SBUF) {
-                    pv_buf = 0;
-                    pv_buf_parity ^= 1u;
-                }
+                for (int kk = 0; kk < AT_KEYS / 32; ++kk)             // 16 keys per MMA: 8 columns of P
+                    at_mma_ts(tmem_o + 128 * half, p_addr + 64 * half + 8 * kk, vd + v_step[AT_KEYS / 32 * half + kk], idesc,
+                              (j | kk) != 0);
+                at_commit(&sh.pv_done[half][j & 1]);
             }
         }
     } else {
         // ---------------- softmax and epilogue: two threads per tile row. Warps w and w + 4 reach the same
-        // quarter of tensor memory; thread `row` of half `part` owns keys 64 part .. 64 part + 63 of its row
-        // in every chunk and columns 64 part .. 64 part + 63 of O. The halves exchange their maxima through
-        // shared memory once a chunk (a barrier of the 256 softmax threads) and their sums once at the end.
-        // With two warps per scheduler one's tensor-memory loads and exponentials run under the other's.
-        __shared__ float half_max[2][2][AT_ROWS], half_sum[2][AT_ROWS];
+        // quarter of tensor memory; thread `row` of half `part` owns keys 64 part .. 64 part + 63 of its row in
+        // every chunk, with a reference maximum, a sum and an O of its own: the halves are two softmaxes over
+        // disjoint keys that meet once, after the last chunk. Nothing ties them together on the way (exchanging
+        // the maxima through a barrier a chunk: 2,500 cycles a chunk, without it 2,050).
+        __shared__ float half_max[2][AT_ROWS], half_sum[2][AT_ROWS];
         const int part = warp >> 2, row = tid & (AT_ROWS - 1);
         const int t_in = row / p.group, h_in = row - t_in * p.group;
         const bool valid = row < p.tokens_per_tile * p.group && t_in < n_tok;
         const int pos = valid ? ctx + tok0 + t_in : -1;                 // -1: every key is masked
         const int lo = first_visible_key(pos, p.window);
         const unsigned lane_base = (unsigned)(32 * (warp & 3)) << 16;
+        const unsigned o_addr = tmem_o + 128 * part + lane_base;
         // distance bias of the row's head; a row that belongs to no token takes none (its scores stay numbers)
         const float r1 = BIASED && valid ? p.distance[kh * p.group + h_in] : 0.f;
         const float r2 = BIASED && valid ? p.distance[p.n_heads + kh * p.group + h_in] : 0.f;
         float m_ref = -INFINITY, l_run = 0.f;
         bool alive = true;
-        // Phases of the "P V done" barrier are consumed strictly in order (phase j completes when the
-        // P V of chunk j has run); the barrier can never be more than one phase ahead of a warp that
-        // has consumed every phase below j - 1 when it starts chunk j, so a parity is never ambiguous.
+        // Phases of the "P V done" barriers are consumed strictly in order (phase j completes when this half's
+        // P V of chunk j has run); they can never be more than one phase ahead of a warp that has consumed
+        // every phase below j - 1 when it starts chunk j, so a parity is never ambiguous.
         int consumed = 0;
         auto pv_consumed_through = [&](int phases) {
             while (alive && consumed < phases) {
-                alive = at_wait(&sh.pv_done[consumed & 1], (unsigned)(consumed >> 1) & 1, p.status);
+                alive = at_wait(&sh.pv_done[part][consumed & 1], (unsigned)(consumed >> 1) & 1, p.status);
                 ++consumed;
             }
         };
-        // A thread whose wait ran out keeps walking the loop without touching anything, so that every
-        // barrier below is reached by all 256 threads; they leave together after the next exchange.
+        // A warp whose wait ran out keeps walking the loop without touching anything, so that the barriers of
+        // the last chunk and of the end are reached by all.
         for (int j = 0; j < n_chunks; ++j) {
             const int b = j % AT_SBUF, s = j % AT_STAGES;
             if (alive) alive = at_wait(&sh.s_full[b], (unsigned)(j / AT_SBUF) & 1, p.status);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             pv_consumed_through(j - 1);               // long completed: this only keeps the count in step
             alive = __all_sync(0xffffffffu, alive);   // the tensor-memory accesses below are warp-wide
-            if (!alive) *reinterpret_cast<volatile int*>(&sh.abort) = 1;
             const int c0 = chunk_of(j) * AT_KEYS, k0 = c0 + 64 * part;
             // rows that belong to no token of the tile need no mask: whatever they compute is never stored,
             // and a row's output depends on that row alone
             const bool edge = __any_sync(0xffffffffu, valid && (k0 + 63 > pos || k0 < lo));
-            const unsigned s_addr = tmem_base + (unsigned)b * 128 + lane_base;
+            const unsigned s_addr = tmem_base + (unsigned)b * 128 + 64 * part + lane_base;
             float sc[64];
             float mx = -INFINITY;
             if (alive) {
-                tmem_load32(s_addr + 64 * part, sc);
-                tmem_load32(s_addr + 64 * part + 32, sc + 32);
+                tmem_load32(s_addr, sc);
+                tmem_load32(s_addr + 32, sc + 32);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
                 if (p.cap_log2 > 0.f) {
                     // small arguments (the usual case) take the polynomial on the FMA pipe; one large score among
@@ -532,15 +530,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                 }
                 mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
             }
-            half_max[j & 1][part][row] = mx;
-            // both halves have their scores in registers from here on: P may overwrite the other half's columns
-            asm volatile("bar.sync 3, 256;\n" ::: "memory");
-            if (*reinterpret_cast<volatile int*>(&sh.abort)) {
-                alive = false;
-                break;                                  // all 256 threads see the flag after the barrier
-            }
             const float scale_log2 = p.cap_log2 > 0.f || BIASED ? 1.f : p.scale_log2;
-            mx = fmaxf(mx, half_max[j & 1][part ^ 1][row]) * scale_log2;
+            mx *= scale_log2;
             const bool jump = mx > m_ref + AT_JUMP || (m_ref == -INFINITY && mx > -INFINITY);
             const float m_new = jump ? mx : m_ref;
             // O may only be touched while no P V is running: the rare rescaling waits for the previous one
@@ -552,13 +543,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                     const float alpha = jump ? at_exp2(m_ref - m_new) : 1.f;     // exp2(-inf) = 0: O was 0 anyway
                     l_run *= alpha;
 #pragma unroll
-                    for (int piece = 0; piece < 2; ++piece) {
+                    for (int piece = 0; piece < 4; ++piece) {
                         float o[32];
-                        tmem_load32(tmem_o + lane_base + 64 * part + 32 * piece, o);
+                        tmem_load32(o_addr + 32 * piece, o);
                         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
                         for (int c = 0; c < 32; ++c) o[c] *= alpha;
-                        tmem_store32(tmem_o + lane_base + 64 * part + 32 * piece, o);
+                        tmem_store32(o_addr + 32 * piece, o);
                     }
                     asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                 }
@@ -567,8 +558,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                 m_ref = m_new;
                 const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
                 float sum0 = 0.f, sum1 = 0.f;
-                // P as bfloat16 pairs over the first 64 columns of this chunk's S buffer: this half's 64 keys
-                // are columns 32 part .. 32 part + 31
+                // P as bfloat16 pairs over the first 32 of this half's 64 columns of the S buffer
                 unsigned packed[32];
 #pragma unroll
                 for (int c = 0; c < 32; ++c) {
@@ -578,62 +568,89 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
                     sum1 += e1;
                     packed[c] = at_pack(e0, e1);
                 }
-                tmem_store32_bits(s_addr + 32 * part, packed);
+                tmem_store32_bits(s_addr, packed);
                 asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                 l_run += sum0 + sum1;
             }
             if (j == n_chunks - 1 && c0 + AT_KEYS - 1 > hi_tile) {
-                // value slots beyond the newest key hold no data yet: zero them in the stage
+                // value slots beyond the newest key hold no data yet: zero this half's in the stage, a row of V^T
+                // (a dim) a thread, eight keys (16 bytes) at a time (an element at a time, with its place found by
+                // divisions, took up to 6 us a tile)
                 if (alive) alive = at_wait(&sh.v_full[s], (unsigned)(j / AT_STAGES) & 1, p.status);
-                unsigned char* vs = v_stage + (size_t)s * 2 * AT_TILE;
+                unsigned char* vs = v_stage + (size_t)s * 2 * AT_TILE + row * p.page_size * 2;
                 const int first_bad = hi_tile + 1 - c0;                     // first key column without data
-                const int row_bytes = p.page_size * 2;
-                for (int item = tid; alive && item < AT_HD * (AT_KEYS - first_bad); item += AT_SOFTMAX_THREADS) {
-                    const int d = item / (AT_KEYS - first_bad), col = first_bad + item % (AT_KEYS - first_bad);
+#pragma unroll
+                for (int c8 = 0; c8 < 8; ++c8) {
+                    const int col = 64 * part + 8 * c8;
+                    if (!alive || col + 8 <= first_bad) continue;
                     const int pg = col >> p.page_shift, kcol = col & (p.page_size - 1);
-                    // 16-byte chunk kcol / 8 of row d, moved by the 32- or 64-byte swizzle of the tile
-                    const int moved = p.page_size == 16 ? ((kcol >> 3) ^ ((d >> 2) & 1)) : ((kcol >> 3) ^ ((d >> 1) & 3));
-                    *reinterpret_cast<__nv_bfloat16*>(vs + (size_t)pg * page_bytes + d * row_bytes + moved * 16 +
-                                                      (kcol & 7) * 2) = __float2bfloat16_rn(0.f);
+                    // 16-byte chunk kcol / 8 of the row, moved by the 32- or 64-byte swizzle of the tile
+                    const int moved = p.page_size == 16 ? ((kcol >> 3) ^ ((row >> 2) & 1)) : ((kcol >> 3) ^ ((row >> 1) & 3));
+                    uint4* at = reinterpret_cast<uint4*>(vs + (size_t)pg * page_bytes + moved * 16);
+                    uint4 keep = make_uint4(0u, 0u, 0u, 0u);
+                    const int good = first_bad - col;                       // of these eight, the first `good` are data
+                    if (good > 0) {
+                        keep = *at;
+                        unsigned* word = reinterpret_cast<unsigned*>(&keep);
+#pragma unroll
+                        for (int w = 0; w < 4; ++w)
+                            word[w] &= (2 * w < good ? 0x0000ffffu : 0u) | (2 * w + 1 < good ? 0xffff0000u : 0u);
+                    }
+                    *at = keep;
                 }
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // ordinary stores, read by the MMA
-                asm volatile("bar.sync 2, 256;\n" ::: "memory");            // all eight softmax warps zeroed their part
+                // all four warps of the half zeroed their rows
+                if (part == 0) asm volatile("bar.sync 2, 128;\n" ::: "memory");
+                else asm volatile("bar.sync 3, 128;\n" ::: "memory");
+                alive = __all_sync(0xffffffffu, alive);
             }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
-            if (lane == 0 && alive) at_arrive(&sh.p_full[b]);
+            if (lane == 0 && alive) at_arrive(&sh.p_full[part][b]);
         }
         pv_consumed_through(n_chunks);
-        // the row's sum of weights: both halves hold a part
+        // the halves meet: each row's two maxima and sums, then each thread joins 64 columns of the two O
+        half_max[part][row] = m_ref;
         half_sum[part][row] = l_run;
-        asm volatile("bar.sync 3, 256;\n" ::: "memory");
-        l_run += half_sum[part ^ 1][row];
         alive = __all_sync(0xffffffffu, alive);
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        if (!alive) *reinterpret_cast<volatile int*>(&sh.abort) = 1;
+        asm volatile("bar.sync 4, 256;\n" ::: "memory");
+        if (*reinterpret_cast<volatile int*>(&sh.abort)) alive = false;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const float m0 = half_max[0][row], m1 = half_max[1][row];
+        m_ref = fmaxf(m0, m1);
+        // a half that saw no key has weight 0 and an O of zeros (its P were zeros)
+        const float w0 = m0 == -INFINITY ? 0.f : at_exp2(m0 - m_ref), w1 = m1 == -INFINITY ? 0.f : at_exp2(m1 - m_ref);
+        l_run = half_sum[0][row] * w0 + half_sum[1][row] * w1;
+        auto joined = [&](int piece, float* o) {
+            float other[32];
+            tmem_load32(tmem_o + lane_base + 64 * part + 32 * piece, o);
+            tmem_load32(tmem_o + 128 + lane_base + 64 * part + 32 * piece, other);
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < 32; ++c) o[c] = fmaf(o[c], w0, other[c] * w1);
+        };
         if (alive && p.n_splits > 1) {
             // a share of the keys: the unnormalised sums, the reference maximum and the sum of weights
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const size_t base = ((size_t)(q_start + tok0 + t_in) * p.n_heads + (size_t)(kh * p.group + h_in)) *
                                     p.n_splits + blockIdx.z;
-            const bool any = n_chunks > 0 && l_run > 0.f;
+            const bool any = l_run > 0.f;
             if (valid && part == 0) {
                 p.part_ml[base * 2] = any ? m_ref * 0.6931471805599453f : -INFINITY;
                 p.part_ml[base * 2 + 1] = any ? l_run : 0.f;
             }
-            if (n_chunks > 0) {                                          // warp-uniform: tensor memory holds sums
 #pragma unroll
-                for (int piece = 0; piece < 2; ++piece) {
-                    float o[32];
-                    tmem_load32(tmem_o + lane_base + 64 * part + 32 * piece, o);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                    if (valid && any) {
-                        float4* dst4 = reinterpret_cast<float4*>(p.part_o + base * AT_HD + 64 * part + 32 * piece);
+            for (int piece = 0; piece < 2; ++piece) {
+                float o[32];
+                joined(piece, o);
+                if (valid && any) {
+                    float4* dst4 = reinterpret_cast<float4*>(p.part_o + base * AT_HD + 64 * part + 32 * piece);
 #pragma unroll
-                        for (int c = 0; c < 32; c += 4) dst4[c / 4] = make_float4(o[c], o[c + 1], o[c + 2], o[c + 3]);
-                    }
+                    for (int c = 0; c < 32; c += 4) dst4[c / 4] = make_float4(o[c], o[c + 1], o[c + 2], o[c + 3]);
                 }
             }
         } else if (alive) {
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             // the sink counts once in the denominator (the reference maximum is in units of log2)
             const float extra = (p.sink && valid && l_run > 0.f)
                                     ? at_exp2(p.sink[kh * p.group + h_in] * 1.4426950408889634f - m_ref) : 0.f;
@@ -643,8 +660,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
 #pragma unroll
             for (int piece = 0; piece < 2; ++piece) {
                 float o[32];
-                tmem_load32(tmem_o + lane_base + 64 * part + 32 * piece, o);
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                joined(piece, o);
                 if (valid) {
 #pragma unroll
                     for (int c = 0; c < 32; c += 8)
@@ -763,6 +779,7 @@ extern "C" int mx_paged_attention_tc_split(const void* q, int q_stride, const vo
     p.sink = sink;
     p.distance = distance;
     p.n_splits = n_splits;
+    p.n_tiles = n_tiles;
     p.part_o = scratch;
     p.part_ml = scratch ? scratch + (size_t)n_tokens * n_heads * n_splits * AT_HD : nullptr;
     const size_t smem = (size_t)(2 + 2 * AT_STAGES * 2) * AT_TILE + 1024;
@@ -774,7 +791,8 @@ extern "C" int mx_paged_attention_tc_split(const void* q, int q_stride, const vo
         if (e != cudaSuccess) MX_REFUSE("tcgen05 attention: cannot reserve %zu bytes of shared memory", smem);
         attribute_set = true;
     }
-    const dim3 grid(n_tiles, n_kv_heads, n_splits);
+    if ((long long)n_tiles * n_kv_heads > 0x7fffffffLL) MX_REFUSE("tcgen05 attention: %d tiles exceed the grid", n_tiles);
+    const dim3 grid((unsigned)(n_tiles * n_kv_heads), 1, n_splits);
     if (distance) attention_tc_kernel<true><<<grid, AT_THREADS, smem, stream>>>(q_map, k_map, v_map, p);
     else attention_tc_kernel<false><<<grid, AT_THREADS, smem, stream>>>(q_map, k_map, v_map, p);
     const int rc = mx_launch_status();
