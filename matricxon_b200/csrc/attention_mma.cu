@@ -66,7 +66,7 @@ struct MmaAttnParams {
     int* status;
     long long n_pages;
     int n_tiles, q_stride, out_stride, bt_stride;
-    int n_heads, n_kv_heads, page_size, page_shift, window, n_splits;
+    int n_heads, n_kv_heads, group, page_size, page_shift, window, n_splits;
     int keep_first;              // with a window: keys j < keep_first stay visible whatever the distance
     float scale_log2;            // scale * log2(e)
     // capped scores: cap_log2 = cap * log2(e) > 0 turns score * scale into cap * tanh(score * scale / cap)
@@ -185,6 +185,51 @@ __device__ __forceinline__ void issue_chunk(const MmaAttnParams& p, __nv_bfloat1
         }
 }
 
+// The same by one warp for narrow tiles, a lane a page: a decode step's attention is a chain of latencies, and one lane
+// that walks the pages and issues every copy took as long as the chunk's arithmetic (2,000 cycles; with this and the
+// divisions by the group taken out of a one-token tile's way, one request at 3,100 tokens of the 3B sizes decodes in
+// 1.64 instead of 1.68 ms a step). Merging the key splits as a cluster of blocks, without the kernel that follows, gained
+// nothing more: clusters of eight that fill an SM each find room for fifteen at a time, and those of smaller blocks
+// started 20 us later.
+template <int HD>
+__device__ __forceinline__ void issue_chunk_warp(const MmaAttnParams& p, __nv_bfloat16* ks, __nv_bfloat16* vs,
+                                                 unsigned long long* bar, int c0, int lo, int hi, int kept, const int* bt,
+                                                 const __nv_bfloat16* kbase, const __nv_bfloat16* vbase,
+                                                 size_t page_stride, int lane, const int* cached) {
+    const int ps = p.page_size, pages = CHUNK >> p.page_shift;
+    const unsigned tile_bytes = (unsigned)(ps * HD * sizeof(__nv_bfloat16));
+    int page = -1;
+    if (lane < pages) {
+        const int key0 = c0 + lane * ps;
+        if (key0 <= hi && (key0 + ps - 1 >= lo || key0 < kept)) {
+            const int lp = key0 >> p.page_shift;
+            page = cached != nullptr ? cached[lane] : (lp < p.bt_stride ? bt[lp] : -1);
+            if (page < 0 || page >= p.n_pages) {
+                page = -1;
+                atomicOr(p.status, MX_STATUS_BAD_PAGE);
+            }
+        }
+    }
+    const unsigned valid = __ballot_sync(0xffffffffu, page >= 0);
+    if (lane == 0) mbar_expect_tx(bar, 2 * tile_bytes * __popc(valid));
+    __syncwarp();
+    if (page >= 0) {
+        bulk_copy(ks + (size_t)lane * ps * HD, kbase + (size_t)page * page_stride, tile_bytes, bar);
+        bulk_copy(vs + (size_t)lane * ps * HD, vbase + (size_t)page * page_stride, tile_bytes, bar);
+    }
+    if (__popc(valid) != pages) {
+        for (int pg = 0; pg < pages; ++pg) {
+            if (valid >> pg & 1) continue;
+            uint4* kz = reinterpret_cast<uint4*>(ks + (size_t)pg * ps * HD);
+            uint4* vz = reinterpret_cast<uint4*>(vs + (size_t)pg * ps * HD);
+            for (int i = lane; i < (int)(tile_bytes / 16); i += 32) {
+                kz[i] = make_uint4(0, 0, 0, 0);
+                vz[i] = make_uint4(0, 0, 0, 0);
+            }
+        }
+    }
+}
+
 struct One { static constexpr int value = 1; };
 struct Two { static constexpr int value = 2; };
 
@@ -213,7 +258,7 @@ attention_mma_kernel(const MmaAttnParams p) {
         const int* row = p.block_tables + (size_t)seq * p.bt_stride;
         for (int e = threadIdx.x; e < min(p.bt_stride, NARROW_TABLE); e += blockDim.x) narrow_table[e] = row[e];
     }
-    const int group = p.n_heads / p.n_kv_heads;
+    const int group = p.group;
     const int q_start = p.cu_q[seq];
     const int q_len = p.cu_q[seq + 1] - q_start;
     const int ctx = p.context_lens[seq];
@@ -227,6 +272,9 @@ attention_mma_kernel(const MmaAttnParams p) {
     }
     __syncthreads();
 
+    // the token of a row; a decoding sequence brings one (no divisions on its way)
+    const bool one_token = NARROW && q_len == 1;
+    auto token_of = [&](int r) { return one_token ? 0 : r / group; };
     // rows of this block and of this warp
     const int tile_last = min(tile_row0 + TILE_ROWS - 1, n_rows - 1);
     const int row0 = NARROW ? tile_row0 : tile_row0 + 16 * warp;
@@ -240,7 +288,7 @@ attention_mma_kernel(const MmaAttnParams p) {
         const int r = row0 + g + 8 * i;
         r_valid[i] = r < n_rows;
         const int rr = r_valid[i] ? r : tile_last;
-        r_tok[i] = rr / group;
+        r_tok[i] = token_of(rr);
         r_head[i] = rr - r_tok[i] * group;
         r_pos[i] = ctx + r_tok[i];
         r_lo[i] = first_visible_key(r_pos[i], p.window);
@@ -254,12 +302,12 @@ attention_mma_kernel(const MmaAttnParams p) {
         }
     }
     // key range of the block (what is fetched) and of the warp (what it computes)
-    const int hi_tile = ctx + tile_last / group;
-    const int lo_tile = first_visible_key(ctx + tile_row0 / group, p.window);
-    const int hi_warp = warp_has_rows ? ctx + last_row / group : -1;
-    const int lo_warp = first_visible_key(ctx + row0 / group, p.window);
+    const int hi_tile = ctx + token_of(tile_last);
+    const int lo_tile = first_visible_key(ctx + token_of(tile_row0), p.window);
+    const int hi_warp = warp_has_rows ? ctx + token_of(last_row) : -1;
+    const int lo_warp = first_visible_key(ctx + token_of(row0), p.window);
     // rows of the warp see every key of a chunk that lies in [all_lo, all_hi]: no mask needed
-    const int all_hi = warp_has_rows ? ctx + row0 / group : -1;
+    const int all_hi = warp_has_rows ? ctx + token_of(row0) : -1;
     const int all_lo = first_visible_key(hi_warp, p.window);
     const bool rows_full = row0 + 15 < n_rows;
     // keys [0, kept) are seen beside the window's: their chunks that lie wholly before the window's first one
@@ -295,8 +343,8 @@ attention_mma_kernel(const MmaAttnParams p) {
     };
     const bool first_is_old = (chunk_of(my_first) + 1) * CHUNK <= ctx;
     if (NARROW && my_count > 0 && first_is_old)
-        issue_chunk<HD>(p, my_stages, my_stages + CHUNK * HD, &my_bars[0], chunk_of(my_first) * CHUNK, lo_tile,
-                        hi_tile, kept, bt, kbase, vbase, page_stride, lane, 32, cached_for(0));
+        issue_chunk_warp<HD>(p, my_stages, my_stages + CHUNK * HD, &my_bars[0], chunk_of(my_first) * CHUNK, lo_tile,
+                             hi_tile, kept, bt, kbase, vbase, page_stride, lane, cached_for(0));
     // queries and the newest keys and values come from the kernels before this one
     pdl_wait();
     // Q fragments: 16 bytes of each owned row per 32-wide block. A row beyond the tile reads the
@@ -519,15 +567,15 @@ attention_mma_kernel(const MmaAttnParams p) {
         // warps a block has eight chunks in flight, and a warp fetches its next chunk when it is done with
         // the one before (more warps hide the copies' latency better than deeper per-warp pipelines did)
         if (my_count > 0 && !first_is_old)
-            issue_chunk<HD>(p, my_stages, my_stages + CHUNK * HD, &my_bars[0], chunk_of(my_first) * CHUNK, lo_tile,
-                            hi_tile, kept, bt, kbase, vbase, page_stride, lane, 32, cached_for(0));
+            issue_chunk_warp<HD>(p, my_stages, my_stages + CHUNK * HD, &my_bars[0], chunk_of(my_first) * CHUNK, lo_tile,
+                                 hi_tile, kept, bt, kbase, vbase, page_stride, lane, cached_for(0));
         for (int i = 0; i < my_count; ++i) {
             const int st = i % NARROW_STAGES;
             if (NARROW_STAGES > 1 && i + 1 < my_count) {
                 const int nx = (i + 1) % NARROW_STAGES;
                 __nv_bfloat16* ks = my_stages + (size_t)nx * STAGE_ELEMS;
-                issue_chunk<HD>(p, ks, ks + CHUNK * HD, &my_bars[nx], chunk_of(my_first + NARROW_WARPS * (i + 1)) * CHUNK,
-                                lo_tile, hi_tile, kept, bt, kbase, vbase, page_stride, lane, 32, cached_for(i + 1));
+                issue_chunk_warp<HD>(p, ks, ks + CHUNK * HD, &my_bars[nx], chunk_of(my_first + NARROW_WARPS * (i + 1)) * CHUNK,
+                                     lo_tile, hi_tile, kept, bt, kbase, vbase, page_stride, lane, cached_for(i + 1));
             }
             __syncwarp();
             mbar_wait(&my_bars[st], (unsigned)((i / NARROW_STAGES) & 1), p.status);
@@ -538,9 +586,9 @@ attention_mma_kernel(const MmaAttnParams p) {
             }
             __syncwarp();                         // the stage may be refilled from here on
             if (NARROW_STAGES == 1 && i + 1 < my_count)
-                issue_chunk<HD>(p, my_stages, my_stages + CHUNK * HD, &my_bars[0],
-                                chunk_of(my_first + NARROW_WARPS * (i + 1)) * CHUNK, lo_tile, hi_tile, kept, bt, kbase, vbase,
-                                page_stride, lane, 32, cached_for(i + 1));
+                issue_chunk_warp<HD>(p, my_stages, my_stages + CHUNK * HD, &my_bars[0],
+                                     chunk_of(my_first + NARROW_WARPS * (i + 1)) * CHUNK, lo_tile, hi_tile, kept, bt, kbase,
+                                     vbase, page_stride, lane, cached_for(i + 1));
         }
         // ---- combine the warps' partial results through shared memory (stages are free)
         __syncthreads();
@@ -591,7 +639,7 @@ attention_mma_kernel(const MmaAttnParams p) {
                 acc.x += v.x * wgt; acc.y += v.y * wgt; acc.z += v.z * wgt; acc.w += v.w * wgt;
             }
             const int row = tile_row0 + r;
-            const int tok = row / group, head = kh * group + (row - tok * group);
+            const int tok = token_of(row), head = kh * group + (row - tok * group);
             if (p.n_splits == 1) {
                 // the sink counts once in the denominator (maxima are in units of log2)
                 const float inv = 1.f / (sum_of[r] + (p.sink ? fast_exp2(p.sink[head] * 1.4426950408889634f - max_of[r]) : 0.f));
@@ -606,7 +654,7 @@ attention_mma_kernel(const MmaAttnParams p) {
         }
         if (p.n_splits > 1 && tid < rows_here) {
             const int row = tile_row0 + tid;
-            const int tok = row / group, head = kh * group + (row - tok * group);
+            const int tok = token_of(row), head = kh * group + (row - tok * group);
             const size_t base = ((size_t)(q_start + tok) * p.n_heads + head) * p.n_splits + split;
             p.part_ml[base * 2] = max_of[tid] * ln2;     // the merge kernel works with natural logs
             p.part_ml[base * 2 + 1] = sum_of[tid];
@@ -739,6 +787,7 @@ extern "C" int mx_paged_attention_mma(const void* q, int q_stride, const void* c
     p.out_stride = out_stride; p.bt_stride = bt_stride; p.n_heads = n_heads; p.n_kv_heads = n_kv_heads;
     p.page_size = page_size; p.page_shift = page_size == 8 ? 3 : (page_size == 16 ? 4 : 5);
     p.window = window; p.n_splits = n_splits;
+    p.group = n_heads / n_kv_heads;
     p.keep_first = window > 0 ? max(keep_first, 0) : 0;
     p.scale_log2 = scale * 1.4426950408889634f;
     p.cap_log2 = softcap > 0.f ? softcap * 1.4426950408889634f : 0.f;
