@@ -14,7 +14,7 @@ Backends, chosen by the runtime:
   "auto"    -- "simt" for float32; for bfloat16 "skinny" up to 16 rows, "tcgen05" above 256 rows,
                "library" between (a weight stream that 128-row tiles would leave to a few SMs) and
                for shapes neither takes (a K that is no multiple of 8), and "stream" from 9 rows
-               on where every SM owns many weight rows (``_pick`` gives the measured thresholds).
+               on for large matrices (``_pick`` gives the measured thresholds).
 """
 
 from __future__ import annotations
@@ -63,13 +63,22 @@ def _pick(x: torch.Tensor, weight: torch.Tensor, m: int, n: int) -> str:
     """The backend "auto" stands for, from measurements on B200 with weights streaming from HBM.
     Up to 8 rows the 16-row kernel is the fastest on every shape (its many small blocks hide the
     latencies that the streaming kernel's one pipeline per SM has to sit through). From 9 rows on that
-    kernel works on two token blocks and slows by 40 %; the streaming kernel does not, and wins where
-    every SM owns enough weight rows to keep its pipeline busy: 64 for 9 to 16 rows (the wide
-    feed-forward matrix: 17 against 23 us; the vocabulary-sized head: 53 against 71 us), 256 for 17 to
-    128 rows (the head: 59 against 66 us for the library's product plus the epilogue kernel)."""
+    kernel works on two token blocks, whose registers leave an SM two blocks of threads instead of three,
+    and is the faster one only while all its blocks run at a time (16 rows: 30.7 against 35.7 us for
+    4608 x 18432, 288 blocks; 17.8 against 14.6 for 5632 x 4608, 352; 74 against 52 for 6144 x 24576, 384;
+    25.7 against 23.6 for 3072 x 12288, 384 with K in two halves; sixteen requests decoding at the 3B sizes
+    2.40 -> 2.12 ms a step against a limit of 64 weight rows per SM). For 17 to 128 rows the streaming kernel
+    wins where every SM owns 256 weight rows (the head: 59 against 66 us for the library's product plus
+    the epilogue kernel)."""
     if 9 <= m <= 128 and kernels.stream_gemm_supported(x, weight):
-        rows_per_block = -(-n // kernels.sm_count(x.device))
-        if rows_per_block >= (64 if m <= 16 else 256):
+        sms = kernels.sm_count(x.device)
+        if m <= 16:
+            blocks = -(-n // 16)
+            if 2 * blocks <= 3 * sms and x.shape[1] % 64 == 0 and x.shape[1] >= 6144:
+                blocks *= 2                       # the kernel shares K between two blocks (mx_gemm_skinny)
+            if blocks > 2 * sms:
+                return "stream"
+        elif -(-n // sms) >= 256:
             return "stream"
     if kernels.skinny_gemm_supported(x, weight):
         return "skinny"
