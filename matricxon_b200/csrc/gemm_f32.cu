@@ -144,7 +144,7 @@ gemm_f32_rows_kernel(const float* __restrict__ A, int lda, const float* __restri
 // 56 rows x 256 features with 7 x 16 outputs a thread, two blocks an SM, 2.36; 64 x 192 unpacked 3.04; the general
 // kernel 4.3.
 constexpr int FT_M = 64, FT_N = 128, FT_K = 16, FT_THREADS = 128;
-constexpr int FT_LDA = 2 * FT_M + 4, FT_LDW = FT_N + 4;          // floats from one k to the next
+constexpr int FT_LDA = FT_M + 4, FT_LDW = FT_N + 4;              // floats from one k to the next
 constexpr int FT_BUFFER = FT_K * (FT_LDA + FT_LDW);
 constexpr int FT_OUT_LD = FT_N + 4;
 constexpr int FT_FLOATS = 2 * FT_BUFFER > FT_M * FT_OUT_LD ? 2 * FT_BUFFER : FT_M * FT_OUT_LD;
@@ -154,7 +154,13 @@ __device__ __forceinline__ void fma_pair(pair_t& acc, pair_t a, pair_t b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-__global__ void __cluster_dims__(F32_PIECES, 1, 1) __launch_bounds__(FT_THREADS, 3)
+__device__ __forceinline__ pair_t both(float v) {
+    pair_t p;
+    asm("mov.b64 %0, {%1, %1};\n" : "=l"(p) : "f"(v));
+    return p;
+}
+
+__global__ void __cluster_dims__(F32_PIECES, 1, 1) __launch_bounds__(FT_THREADS, 4)
 gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw,
                      const float* __restrict__ bias, const float* residual, float* out, int ldo, int M, int N, int K,
                      int piece, int mode) {
@@ -164,8 +170,8 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
     const int m0 = (blockIdx.x / F32_PIECES) * FT_M, n0 = blockIdx.y * FT_N;
     const int k_begin = min(rank * piece, K), k_end = min(k_begin + piece, K);
     const int steps = (k_end - k_begin + FT_K - 1) / FT_K;
-    // this thread's outputs: rows m_lane + 8 i + {0, 1}, features n_lane + 32 j + {0 .. 3}
-    const int m_lane = (warp & 1) * 32 + 2 * (lane >> 3), n_lane = (warp >> 1) * 64 + 4 * (lane & 7);
+    // this thread's outputs: rows m_lane + 16 i + {0 .. 3}, features n_lane + 32 j + {0 .. 3}
+    const int m_lane = (warp & 1) * 32 + 4 * (lane >> 3), n_lane = (warp >> 1) * 64 + 4 * (lane & 7);
 
     // this thread brings k = col .. col + 3 of rows row + 32 i
     const int col = 4 * (tid & 3), row = tid >> 2;
@@ -196,7 +202,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
             const float v[4] = {next_a[i].x, next_a[i].y, next_a[i].z, next_a[i].w};
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                *reinterpret_cast<float2*>(a + (col + e) * FT_LDA + 2 * ((row + 32 * i) ^ (4 * turn))) = make_float2(v[e], v[e]);
+                a[(col + e) * FT_LDA + ((row + 32 * i) ^ (8 * turn))] = v[e];
         }
 #pragma unroll
         for (int i = 0; i < FT_N / 32; ++i) {
@@ -224,10 +230,12 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
             const int flip = k >> 3;
             pair_t av[8], wv[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(a + k * FT_LDA + 2 * ((m_lane + 8 * i) ^ (4 * flip)));
-                av[2 * i] = v.x;
-                av[2 * i + 1] = v.y;
+            for (int i = 0; i < 2; ++i) {
+                const float4 v = *reinterpret_cast<const float4*>(a + k * FT_LDA + ((m_lane + 16 * i) ^ (8 * flip)));
+                av[4 * i] = both(v.x);
+                av[4 * i + 1] = both(v.y);
+                av[4 * i + 2] = both(v.z);
+                av[4 * i + 3] = both(v.w);
             }
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
@@ -247,7 +255,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int lda, const float* __restri
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j)
-            *reinterpret_cast<ulonglong2*>(smem + (m_lane + 8 * (i >> 1) + (i & 1)) * FT_OUT_LD + n_lane + 32 * j) =
+            *reinterpret_cast<ulonglong2*>(smem + (m_lane + 16 * (i >> 2) + (i & 3)) * FT_OUT_LD + n_lane + 32 * j) =
                 make_ulonglong2(acc[i][2 * j], acc[i][2 * j + 1]);
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
