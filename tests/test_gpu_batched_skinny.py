@@ -36,3 +36,32 @@ def test_interleaved_members(m, n, k_dim, dtype):
     alone = torch.empty(1, batch, n, device=DEV, dtype=dtype)
     k.gemm_batched_skinny(a[m - 1:m], w, alone)
     assert torch.equal(alone[0], out[m - 1])             # a row's result does not depend on the others
+
+
+@pytest.mark.parametrize("k_dim", [128, 512])
+def test_weights_that_the_kernel_before_wrote(k_dim):
+    """Chained launches: the product may be on the GPU before the norm that writes its weights has ended."""
+    from matricxon_b200.ops import kernels as k
+
+    torch.manual_seed(k_dim)
+    batch, n, rounds = 16, 128, 12
+    a = torch.randn(4, batch, k_dim, device=DEV).bfloat16()
+    xs = [torch.randn(batch * n, k_dim, device=DEV) for _ in range(rounds)]
+    scale = torch.ones(k_dim, device=DEV)
+    w = torch.zeros(batch * n, k_dim, device=DEV, dtype=torch.bfloat16)
+    outs = [torch.empty(4, batch, n, device=DEV) for _ in range(rounds)]
+    kept = [torch.empty_like(w) for _ in range(rounds)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):                            # back to back, with nothing of the host's in between
+        for x, out, copy in zip(xs, outs, kept):
+            k.rmsnorm(x, scale, 0.0, 1e-6, w)
+            k.gemm_batched_skinny(a, w.view(batch, n, k_dim), out)
+            copy.copy_(w)
+    graph.replay()
+    torch.cuda.synchronize()
+    for x, out, copy in zip(xs, outs, kept):
+        members = copy.double().view(batch, n, k_dim)
+        exact = torch.einsum("mbk,bnk->mbn", a.double(), members)
+        bound = (k_dim * 2.0 ** -24) * torch.einsum("mbk,bnk->mbn", a.double().abs(), members.abs())
+        assert bool(((out.double() - exact).abs() <= bound + 1e-30).all())
+        assert bool((copy.float() - x / x.pow(2).mean(dim=1, keepdim=True).sqrt()).abs().max() < 0.05)
