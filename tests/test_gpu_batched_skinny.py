@@ -65,3 +65,37 @@ def test_weights_that_the_kernel_before_wrote(k_dim):
         bound = (k_dim * 2.0 ** -24) * torch.einsum("mbk,bnk->mbn", a.double().abs(), members.abs())
         assert bool(((out.double() - exact).abs() <= bound + 1e-30).all())
         assert bool((copy.float() - x / x.pow(2).mean(dim=1, keepdim=True).sqrt()).abs().max() < 0.05)
+
+
+@pytest.mark.parametrize("k_dim", [32, 128, 512])
+def test_float_results_are_as_good_as_multiply_adds(k_dim):
+    """Against 64 bits no further off than one rounding a product and one an addition of the lanes' tree gave."""
+    from matricxon_b200.ops import kernels as k
+
+    torch.manual_seed(k_dim)
+    batch, n = 16, 128
+    a = torch.randn(16, batch, k_dim, device=DEV).bfloat16()
+    w = torch.randn(batch, n, k_dim, device=DEV).bfloat16()
+    out = torch.empty(16, batch, n, device=DEV)
+    k.gemm_batched_skinny(a, w, out)
+    exact = torch.einsum("mbk,bnk->mbn", a.double(), w.double())
+    # A rounding is 0.40 units of 2^-24 on average (uniform within half a last place, over all mantissas). Sums are added in
+    # pairs, so each level's roundings together are one such error of the whole sum, and above products of 16 k there
+    # are at most eight levels (512 long): sqrt(8) x 0.40 = 1.13. One chain of the tensor cores' own additions: 2.1.
+    off = float((out.double() - exact).norm() / exact.norm())
+    assert off <= 1.15 * 2.0 ** -24, off * 2.0 ** 24
+
+
+def test_infinities_and_nan_stay_in_their_rows():
+    from matricxon_b200.ops import kernels as k
+
+    for dtype in (torch.float32, torch.bfloat16):
+        a, w = torch.randn(5, 2, 64, device=DEV).bfloat16(), torch.randn(2, 20, 64, device=DEV).bfloat16()
+        a[0, 0, 5], a[1, 0, 63], a[2, 1, 0] = math.inf, math.nan, -math.inf
+        out = torch.empty(5, 2, 20, device=DEV, dtype=dtype)
+        k.gemm_batched_skinny(a, w, out)
+        assert torch.equal(out[0, 0].float(), w[0, :, 5].sign().float() * math.inf) and bool(out[1, 0].isnan().all())
+        assert torch.equal(out[2, 1].float(), -w[1, :, 0].sign().float() * math.inf)
+        kept = torch.ones(5, 2, dtype=torch.bool)
+        kept[0, 0] = kept[1, 0] = kept[2, 1] = False
+        assert bool(out[kept.to(DEV)].isfinite().all())
