@@ -20,8 +20,14 @@ namespace {
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 constexpr int THREADS = (BM / TM) * (BN / TN);  // 256
 
+// Bound by latency where a block has an SM to itself and by what shared memory hands to registers where blocks fill the
+// SMs. A k-tile's operands are on their way in registers while the one before is worked on, and the pieces that are done
+// wait in shared memory: 64 registers, four blocks an SM. 389 x 2,048 x 2,047: 166 us, 16 members of 2,048 x 512 x 128:
+// 185, 16 x 2,048 x 2,047: 95 (the pieces in registers, 102 of them, two blocks an SM: 195, 224 and 159; one chain over
+// K in 40 registers without the loads ahead: 238, 179 and 247). Five blocks an SM leave the loads ahead no registers
+// (205, 203 and 159).
 template <typename TIn, typename TOut>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 4)
 gemm_simt_kernel(const TIn* __restrict__ A, const TIn* __restrict__ W,
                  const float* __restrict__ bias, const float* residual, TOut* out,
                  int M, int N, int K, int lda, int ldw, int ldo, int mode,
@@ -37,54 +43,80 @@ gemm_simt_kernel(const TIn* __restrict__ A, const TIn* __restrict__ W,
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int tx = tid % (BN / TN), ty = tid / (BN / TN);
 
-    float acc[TM][TN], first[TM][TN], pair[TM][TN];      // the piece in hand; p0 + p1; p0 or p2
+    float acc[TM][TN];                                   // the piece in hand
+    __shared__ float4 saved[2][TM][THREADS];             // p0, then p0 + p1; p2
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = first[i][j] = pair[i][j] = 0.f;
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
     const int piece = f32_piece(K);
+    int left = piece, ended = 0;                         // k to the end of the piece; pieces behind it
 
-    // each thread stages 4 elements of A and 4 of W per k-tile: row = tid / 4, 4 k's at (tid % 4) * 4
+    // each thread stages 4 elements of A and 4 of W per k-tile: row = tid / 4, 4 k's at (tid % 4) * 4; rows of the upper
+    // eight k are moved by eight floats, so that a warp's writes of four k fall on different banks
     const int lrow = tid >> 2, lk = (tid & 3) << 2;
-    for (int k0 = 0; k0 < K; k0 += BK) {
+    const bool a_in = m0 + lrow < M, w_in = n0 + lrow < N;
+    const TIn* a_row = A + (size_t)(a_in ? m0 + lrow : 0) * lda;
+    const TIn* w_row = W + (size_t)(w_in ? n0 + lrow : 0) * ldw;
+    const int put = lrow ^ (lk & 8);
+    float na[4], nw[4];
+    auto fetch = [&](int k0) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int k = k0 + lk + e;
-            const int am = m0 + lrow, wn = n0 + lrow;
-            As[lk + e][lrow] = (am < M && k < K) ? to_float(A[(size_t)am * lda + k]) : 0.f;
-            Ws[lk + e][lrow] = (wn < N && k < K) ? to_float(W[(size_t)wn * ldw + k]) : 0.f;
+            na[e] = (a_in && k < K) ? to_float(a_row[k]) : 0.f;
+            nw[e] = (w_in && k < K) ? to_float(w_row[k]) : 0.f;
+        }
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < K; k0 += BK) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            As[lk + e][put] = na[e];
+            Ws[lk + e][put] = nw[e];
         }
         __syncthreads();
+        fetch(k0 + BK);
 #pragma unroll
         for (int kk = 0; kk < BK; ++kk) {
             float a[TM], w[TN];
 #pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
+            for (int i = 0; i < TM; ++i) a[i] = As[kk][((ty * TM) ^ (kk & 8)) + i];
 #pragma unroll
-            for (int j = 0; j < TN; ++j) w[j] = Ws[kk][tx * TN + j];
+            for (int j = 0; j < TN; ++j) w[j] = Ws[kk][((tx * TN) ^ (kk & 8)) + j];
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
         }
         __syncthreads();
-        if ((k0 + BK) % piece == 0 && k0 + BK < K) {         // a piece ends (its length is a multiple of BK)
-            const bool second = (k0 + BK) / piece == 2;
+        left -= BK;
+        if (left == 0 && k0 + BK < K) {                      // a piece ends (its length is a multiple of BK)
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) {
-                    if (second) first[i][j] = pair[i][j] + acc[i][j];
-                    pair[i][j] = second ? 0.f : acc[i][j];
-                    acc[i][j] = 0.f;
+            for (int i = 0; i < TM; ++i) {
+                float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+                if (ended == 1) {
+                    const float4 p0 = saved[0][i][tid];
+                    v = make_float4(p0.x + v.x, p0.y + v.y, p0.z + v.z, p0.w + v.w);
                 }
+                saved[ended == 2][i][tid] = v;
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+            }
+            ++ended;
+            left = piece;
         }
     }
     // the last piece that has any k: p0 or p2 stands alone, p1 or p3 joins the one before it
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = first[i][j] + (pair[i][j] + acc[i][j]);
+    for (int i = 0; i < TM; ++i) {
+        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 p2 = ended == 3 ? saved[1][i][tid] : none, sum = ended > 0 ? saved[0][i][tid] : none;
+        acc[i][0] = sum.x + (p2.x + acc[i][0]);
+        acc[i][1] = sum.y + (p2.y + acc[i][1]);
+        acc[i][2] = sum.z + (p2.z + acc[i][2]);
+        acc[i][3] = sum.w + (p2.w + acc[i][3]);
+    }
 
 #pragma unroll
     for (int i = 0; i < TM; ++i) {

@@ -50,3 +50,22 @@ def test_infinities_and_nan_stay_in_their_rows():
         k.gemm_simt(a, w, None, None, out, k.EPILOGUE_F32)
         assert torch.equal(out[0], w[:, 5].sign() * math.inf) and bool(out[1].isnan().all())
         assert bool(out[2:].isfinite().all())
+
+
+# pieces of K: one, one and a short one, three and a short one, four; members interleaved as heads in a row
+@pytest.mark.parametrize("k_dim", [31, 33, 100, 512])
+@pytest.mark.parametrize("m", [1, 64, 130])
+def test_batched_members_give_a_plain_products_bits(m, k_dim):
+    from matricxon_b200.ops import kernels as k
+
+    torch.manual_seed(m * 1000 + k_dim)
+    batch, n = 3, 70
+    a, w = torch.randn(m, batch, k_dim, device=DEV), torch.randn(batch, n, k_dim, device=DEV)
+    bias = torch.randn(batch, n, device=DEV)
+    out = torch.full((m, batch, n + 2), float("nan"), device=DEV)
+    k.gemm_batched_simt(a, w, bias, out[:, :, :n])
+    alone = torch.empty(m, n, device=DEV)
+    for b in range(batch):
+        k.gemm_simt(a[:, b], w[b], bias[b], None, alone, k.EPILOGUE_F32)
+        assert torch.equal(out[:, b, :n], alone), b
+    assert bool(out[:, :, n:].isnan().all())
