@@ -305,8 +305,19 @@ cudaError_t launch_rows(const float* A, int lda, const float* W, int ldw, const 
 
 }  // namespace
 
-bool mx_gemm_f32_takes(const float* A, int lda, const float* W, int ldw, int N, int K) {
-    return K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
+// Both kernels pay for four pieces of K and for filling their rings or clusters, whatever K is: below these lengths the
+// general kernel is the faster one. 2,048 columns, us here against there: 4 rows of 16 k 2.6 and 3.1; 16 of 16, 3.6 and
+// 3.2; 32 of 32, 5.4 and 4.1, of 64, 5.1 and 5.6; 389 of 16, 11.3 and 4.2, of 96, 15.2 and 12.6, of 128, 15.4 and 15.9.
+// 8,192 columns give the streaming kernel's blocks several rows each: 8 rows of 16 k take 4.6 and 3.3. Between 128 and 192
+// the pieces are 64 long and the last block of a cluster has none: 1,024 x 1,024 x 160 takes 22.0 and 17.0.
+extern "C" int mx_gemm_f32_pays(int M, int N, int K) {
+    if (M > F32_FEW_ROWS) return K >= 192 || (K > 96 && K <= 128);
+    const int several = N > 4096 ? 2 : 1;
+    return K >= (M <= 8 ? (several > 1 ? 32 : 0) : M <= 16 ? 32 * several : 64 * several);
+}
+
+bool mx_gemm_f32_takes(const float* A, int lda, const float* W, int ldw, int M, int N, int K) {
+    return mx_gemm_f32_pays(M, N, K) && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
            ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0 && (N + FT_N - 1) / FT_N <= 65535;
 }
 

@@ -11,7 +11,8 @@ constexpr int F32_FEW_ROWS = 32;
 // Length of a piece of K: a quarter, in whole steps of the kernels' loops (the last pieces may be short or empty).
 __host__ __device__ inline int f32_piece(int K) { return ((K + F32_PIECES - 1) / F32_PIECES + 31) / 32 * 32; }
 
-// Whether gemm_f32.cu takes these operands (16-byte reads); it gives the same bits as the general kernel.
-bool mx_gemm_f32_takes(const float* A, int lda, const float* W, int ldw, int N, int K);
+// Whether gemm_f32.cu takes these operands (16-byte reads, and enough of K); it gives the same bits as the general kernel.
+extern "C" int mx_gemm_f32_pays(int M, int N, int K);
+bool mx_gemm_f32_takes(const float* A, int lda, const float* W, int ldw, int M, int N, int K);
 int mx_gemm_f32(const float* A, int lda, const float* W, int ldw, const float* bias, const float* residual, float* out,
                 int ldo, int M, int N, int K, int mode, cudaStream_t stream);

@@ -151,7 +151,7 @@ extern "C" int mx_gemm_simt(const void* A, const void* W, int in_dtype, const fl
                   in_dtype, expected_out, out_dtype);
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) MX_REFUSE("gemm: M = %d is beyond this kernel's grid", M);
-    if (in_dtype == MX_DTYPE_F32 && mx_gemm_f32_takes((const float*)A, lda, (const float*)W, ldw, N, K))
+    if (in_dtype == MX_DTYPE_F32 && mx_gemm_f32_takes((const float*)A, lda, (const float*)W, ldw, M, N, K))
         return mx_gemm_f32((const float*)A, lda, (const float*)W, ldw, bias, residual, (float*)out, ldo, M, N, K, mode, stream);
 #define MX_GEMM(TI, TO) \
     gemm_simt_kernel<TI, TO><<<grid, THREADS, 0, stream>>>((const TI*)A, (const TI*)W, bias, residual, (TO*)out, M, N, K, lda, ldw, ldo, mode, 0, 0, 0, 0)

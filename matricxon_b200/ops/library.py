@@ -35,6 +35,7 @@ _SIGNATURES: dict[str, tuple[list, object]] = {
     "mx_rope_kv_write_bias": ([P, I, I, P, P, P, P, I, I, I, I, I, I, L, I, P, P, P], I),
     "mx_epilogue": ([P, I, P, P, P, I, L, I, I, P], I),
     "mx_gemm_simt": ([P, P, I, P, P, P, I, I, I, I, I, I, I, I, P], I),
+    "mx_gemm_f32_pays": ([I, I, I], I),
     "mx_gemm_tcgen05": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P, P], I),
     "mx_gemm_tcgen05_force_tiles": ([I], I),
     "mx_gemm_stream": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P, P], I),

@@ -1,0 +1,15 @@
+"""Which float products the kernels for few and for many rows take, and which are too short in K for them."""
+
+import pytest
+
+
+@pytest.mark.parametrize("m,n,least", [
+    (1, 2048, 0), (8, 4096, 0), (8, 8192, 32), (9, 2048, 32), (16, 8192, 64), (17, 2048, 64), (32, 8192, 128),
+    (33, 16, 100), (2048, 2048, 100)])
+def test_shortest_k(m, n, least):
+    from matricxon_b200.ops.library import library
+
+    pays = library().mx_gemm_f32_pays
+    assert pays(m, n, least) and (least == 0 or not pays(m, n, least - 4))
+    # a low-rank factor of a prompt stays with the general kernel, and so does a K whose fourth piece would be empty
+    assert not pays(389, 2048, 16) and not pays(389, 2048, 160) and pays(389, 2048, 192)
