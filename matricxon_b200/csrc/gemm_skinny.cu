@@ -80,7 +80,13 @@ struct SkinnyRope {
 // the second hands its sums to the first through distributed shared memory, which adds them after its
 // own (a fixed order) and runs the epilogue. For matrices with so few output features that one block
 // per tile leaves most of the GPU's warp slots, and so most of the loads it could have in flight, unused.
-template <int MB, bool ROPE, bool SPLIT, int UNROLL = SK_UNROLL, bool WIDE = false>
+// GATHER: every load of a trip is out before its first product. Loads do not move across the barrier that says so; without
+// it the assembler spreads them between the products to stay within 72 registers with two blocks of tokens. That costs an
+// SM its third block of threads, so a product whose blocks fit three to an SM but not two goes without
+// (skinny_gathers). 16 rows, gathered and not: 2,048 x 8,192 in 11.2 and 16.8 us, 12,288 x 3,072 in 20.4 and 22.6, but
+// 6,144 x 1,024 in 6.6 and 6.1, 5,632 x 4,608 in 18.6 and 16.9. All weights ahead of all activations, or the other way
+// round, took 20 % longer for up to 8 rows.
+template <int MB, bool ROPE, bool SPLIT, int UNROLL = SK_UNROLL, bool WIDE = false, bool GATHER = true>
 __global__ void __launch_bounds__(SK_THREADS)
 gemm_skinny_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ W,
                    int ldw, const float* __restrict__ bias, const float* residual, void* out,
@@ -167,11 +173,7 @@ gemm_skinny_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bflo
                 for (int h = 0; h < HALVES; ++h)
                     xf[u][mb][h] = (in && tok_ok[mb]) ? load_row(xrow[mb] + PIECE * kb + 8 * h) : make_uint4(0, 0, 0, 0);
         }
-        // Every load of the trip is out before its first product: loads do not move across the barrier. Without it the
-        // assembler spread them between the products to stay within 64 registers with two blocks of tokens (16 rows,
-        // 2048 x 8192: 16.6 us, with it 11.4; one request decoding 1.641 -> 1.637 ms a step). All weights ahead of all
-        // activations, or the other way round, took 20 % longer for up to 8 rows.
-        __syncwarp();
+        if constexpr (GATHER) __syncwarp();
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u)
 #pragma unroll
@@ -307,6 +309,14 @@ bool skinny_deep(int grid, int K) {
     return grid <= 2 * skinny_sm_count() && K / 32 > SK_WARPS * SK_UNROLL;
 }
 
+// Whether a product of 9 to 16 rows keeps its loads together: not where its blocks fit three to an SM but not two. Long
+// rows gather all the same (4,752 x 6,144, 9 rows: 17.7 us gathered, 19.7 not; at K = 4,608, 14.9 and 15.8, but 17.0 and 16.4
+// for 5,632 columns).
+bool skinny_gathers(int M, int grid, int K) {
+    const int sms = skinny_sm_count();
+    return M <= 8 || grid <= 2 * sms || grid > 3 * sms || K > 4608;
+}
+
 // 32-byte loads want pieces of 64 and rows that start on 32-byte boundaries
 bool skinny_wide_ok(const void* W, int K, int ldw) {
     return K % 64 == 0 && ldw % 16 == 0 && reinterpret_cast<uintptr_t>(W) % 32 == 0;
@@ -359,6 +369,7 @@ extern "C" int mx_gemm_skinny(const void* x, const void* W, const float* bias, c
         return MX_OK;
     }
     auto kernel = M <= 8 ? gemm_skinny_kernel<1, false, false> : gemm_skinny_kernel<2, false, false>;
+    if (!skinny_gathers(M, grid, K)) kernel = gemm_skinny_kernel<2, false, false, SK_UNROLL, false, false>;
     if (skinny_deep(grid, K)) {
         // (both row counts: a row's sum is then formed in the same order whatever the batch)
         if (skinny_wide_ok(W, K, ldw))
@@ -393,6 +404,7 @@ extern "C" int mx_gemm_skinny_rope(const void* x, const void* W, const float* bi
     rope.n_heads = n_heads; rope.n_kv_heads = n_kv_heads; rope.head_dim = head_dim; rope.page_size = page_size;
     const int N = (n_heads + 2 * n_kv_heads) * head_dim;
     auto kernel = M <= 8 ? gemm_skinny_kernel<1, true, false> : gemm_skinny_kernel<2, true, false>;
+    if (!skinny_gathers(M, N / 16, K)) kernel = gemm_skinny_kernel<2, true, false, SK_UNROLL, false, false>;
     if (skinny_deep(N / 16, K)) {
         if (skinny_wide_ok(W, K, ldw))
             kernel = M <= 8 ? gemm_skinny_kernel<1, true, false, SK_DEEP / 2, true>
