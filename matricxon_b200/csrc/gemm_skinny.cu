@@ -331,6 +331,14 @@ int check_skinny(int M, int K, int ldx, int ldw) {
 
 }  // namespace
 
+// Blocks of the product of up to 16 rows on n_sm SMs: one a tile of 16 columns, or two (SPLIT) where tiles are few and K is
+// long (c_proj 3072 x 12288: 14.8 us against 16.9; at K = 3072 the halves are too short to pay for the exchange: 6.7
+// against 6.6).
+extern "C" int mx_gemm_skinny_blocks(int N, int K, int n_sm) {
+    const int tiles = (N + 15) / 16;
+    return 2 * tiles <= 3 * n_sm && K % 64 == 0 && K >= 6144 ? 2 * tiles : tiles;
+}
+
 extern "C" int mx_gemm_skinny(const void* x, const void* W, const float* bias, const float* residual,
                               void* out, int out_dtype, int M, int N, int K, int ldx, int ldw, int ldo,
                               int mode, cudaStream_t stream) {
@@ -343,9 +351,7 @@ extern "C" int mx_gemm_skinny(const void* x, const void* W, const float* bias, c
         MX_REFUSE("skinny gemm: epilogue mode %d does not write dtype %d", mode, out_dtype);
     const SkinnyRope none = {};
     const int grid = (N + 15) / 16;
-    if (2 * grid <= 3 * skinny_sm_count() && K % 64 == 0 && K >= 6144) {
-        // few tiles and a long K: two blocks a tile, as a cluster of two (c_proj 3072 x 12288: 14.8 us
-        // against 16.9; at K = 3072 the halves are too short to pay for the exchange: 6.7 against 6.6)
+    if (mx_gemm_skinny_blocks(N, K, skinny_sm_count()) > grid) {     // two blocks a tile, as a cluster of two
         auto kernel = M <= 8 ? gemm_skinny_kernel<1, false, true> : gemm_skinny_kernel<2, false, true>;
         cudaLaunchConfig_t config = {};
         config.gridDim = dim3(2 * grid);

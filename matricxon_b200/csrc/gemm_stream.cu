@@ -260,6 +260,19 @@ int gs_round_up(int v, int to) { return (v + to - 1) / to * to; }
 
 }  // namespace
 
+extern "C" int mx_gemm_skinny_blocks(int N, int K, int n_sm);
+
+// Whether a product of 9 to 16 rows that both kernels take is better off here than on the 16-row kernel: where that
+// kernel's blocks, of which an SM holds two, do not all run at a time, and an SM's share of the weights fills this kernel's
+// ring at least once or is 64 rows and more. 9 and 16 rows, us there against here, weights from HBM: 4,752 x 3,072 11.2 and
+// 11.5 against 11.4 and 11.4, 7,168 x 2,048 9.9 and 10.8 against 9.8 and 10.1, 5,632 x 4,608 16.4 and 16.9 against 14.3 and 14.5,
+// 6,144 x 24,576 74 against 52 at 16; below a ring, 6,144 x 1,024 5.6 and 6.1 against 7.3 and 7.5, 5,120 x 2,048 8.4 and 8.9
+// against 9.7; all blocks at a time, 4,608 x 18,432 30.7 against 35.7 at 16.
+extern "C" int mx_gemm_stream_pays(int N, int K, int n_sm) {
+    return mx_gemm_skinny_blocks(N, K, n_sm) > 2 * n_sm &&
+           (2LL * N * K >= (long long)n_sm * GS_RING_BYTES || (N + n_sm - 1) / n_sm >= 64);
+}
+
 extern "C" int mx_gemm_stream(const void* x, const void* W, const float* bias, const float* residual, void* out,
                               int out_dtype, int M, int N, int K, int ldx, int ldw, int ldo, int mode,
                               int* status, cudaStream_t stream) {

@@ -272,6 +272,11 @@ def stream_gemm_supported(a: torch.Tensor, w: torch.Tensor) -> bool:
             and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def stream_gemm_pays(n: int, k: int, n_sm: int) -> bool:
+    """Whether a product of 9 to 16 rows is better off on the streaming kernel than on the 16-row one (gemm_stream.cu)."""
+    return bool(library().mx_gemm_stream_pays(n, k, n_sm))
+
+
 def gemm_stream(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None,
                 residual: torch.Tensor | None, out: torch.Tensor, mode: int,
                 status: torch.Tensor | None = None) -> None:

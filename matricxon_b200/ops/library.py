@@ -38,6 +38,8 @@ _SIGNATURES: dict[str, tuple[list, object]] = {
     "mx_gemm_f32_pays": ([I, I, I], I),
     "mx_gemm_tcgen05": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P, P], I),
     "mx_gemm_tcgen05_force_tiles": ([I], I),
+    "mx_gemm_stream_pays": ([I, I, I], I),
+    "mx_gemm_skinny_blocks": ([I, I, I], I),
     "mx_gemm_stream": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P, P], I),
     "mx_gemm_skinny": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P], I),
     "mx_gemm_skinny_rope": ([P, P, P, P, I, I, I, I, I, P, P, P, P, L, I, I, I, I, P, P], I),

@@ -62,23 +62,15 @@ def resolve_backend(requested: str, dtype: torch.dtype) -> str:
 def _pick(x: torch.Tensor, weight: torch.Tensor, m: int, n: int) -> str:
     """The backend "auto" stands for, from measurements on B200 with weights streaming from HBM.
     Up to 8 rows the 16-row kernel is the fastest on every shape (its many small blocks hide the
-    latencies that the streaming kernel's one pipeline per SM has to sit through). From 9 rows on that
-    kernel works on two token blocks, whose registers leave an SM two blocks of threads instead of three,
-    and is the faster one only while all its blocks run at a time (16 rows: 30.7 against 35.7 us for
-    4608 x 18432, 288 blocks; 17.8 against 14.6 for 5632 x 4608, 352; 74 against 52 for 6144 x 24576, 384;
-    25.7 against 23.6 for 3072 x 12288, 384 with K in two halves; sixteen requests decoding at the 3B sizes
-    2.40 -> 2.12 ms a step against a limit of 64 weight rows per SM). For 17 to 128 rows the streaming kernel
-    wins where every SM owns 256 weight rows (the head: 59 against 66 us for the library's product plus
-    the epilogue kernel)."""
+    latencies that the streaming kernel's one pipeline per SM has to sit through). For 9 to 16 rows it works on two
+    token blocks, with registers for two blocks of threads an SM, and the streaming kernel takes the products whose
+    blocks do not all run at a time and that are large enough for its pipeline (``kernels.stream_gemm_pays``: sixteen
+    requests decoding at the 3B sizes 2.40 -> 2.12 ms a step against a limit of 64 weight rows per SM). For 17 to 128 rows
+    it wins where every SM owns 256 weight rows (the head: 59 against 66 us for the library's product plus the epilogue
+    kernel)."""
     if 9 <= m <= 128 and kernels.stream_gemm_supported(x, weight):
         sms = kernels.sm_count(x.device)
-        if m <= 16:
-            blocks = -(-n // 16)
-            if 2 * blocks <= 3 * sms and x.shape[1] % 64 == 0 and x.shape[1] >= 6144:
-                blocks *= 2                       # the kernel shares K between two blocks (mx_gemm_skinny)
-            if blocks > 2 * sms:
-                return "stream"
-        elif -(-n // sms) >= 256:
+        if kernels.stream_gemm_pays(n, x.shape[1], sms) if m <= 16 else -(-n // sms) >= 256:
             return "stream"
     if kernels.skinny_gemm_supported(x, weight):
         return "skinny"
