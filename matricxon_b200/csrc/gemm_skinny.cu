@@ -84,7 +84,7 @@ struct SkinnyRope {
 // it the assembler spreads them between the products to stay within 72 registers with two blocks of tokens. That costs an
 // SM its third block of threads, so a product whose blocks fit three to an SM but not two goes without
 // (skinny_gathers). 16 rows, gathered and not: 2,048 x 8,192 in 11.2 and 16.8 us, 12,288 x 3,072 in 20.4 and 22.6, but
-// 6,144 x 1,024 in 6.6 and 6.1, 5,632 x 4,608 in 18.6 and 16.9. All weights ahead of all activations, or the other way
+// 6,144 x 1,024 in 6.6 and 6.1, 5,120 x 2,048 in 9.5 and 8.9. All weights ahead of all activations, or the other way
 // round, took 20 % longer for up to 8 rows.
 template <int MB, bool ROPE, bool SPLIT, int UNROLL = SK_UNROLL, bool WIDE = false, bool GATHER = true>
 __global__ void __launch_bounds__(SK_THREADS)
@@ -310,8 +310,9 @@ bool skinny_deep(int grid, int K) {
 }
 
 // Whether a product of 9 to 16 rows keeps its loads together: not where its blocks fit three to an SM but not two. Long
-// rows gather all the same (4,752 x 6,144, 9 rows: 17.7 us gathered, 19.7 not; at K = 4,608, 14.9 and 15.8, but 17.0 and 16.4
-// for 5,632 columns).
+// rows gather all the same (4,752 x 6,144, 9 rows: 17.7 us gathered, 19.7 not), and so does the QKV product with rotation:
+// 352 blocks and K = 4,608, a step of ten requests at the 7B sizes takes 988 to 999 us gathered and 996 to 1,000 not, of
+// sixteen 1,008 to 1,024 and 1,006 to 1,008.
 bool skinny_gathers(int M, int grid, int K) {
     const int sms = skinny_sm_count();
     return M <= 8 || grid <= 2 * sms || grid > 3 * sms || K > 4608;
@@ -410,7 +411,6 @@ extern "C" int mx_gemm_skinny_rope(const void* x, const void* W, const float* bi
     rope.n_heads = n_heads; rope.n_kv_heads = n_kv_heads; rope.head_dim = head_dim; rope.page_size = page_size;
     const int N = (n_heads + 2 * n_kv_heads) * head_dim;
     auto kernel = M <= 8 ? gemm_skinny_kernel<1, true, false> : gemm_skinny_kernel<2, true, false>;
-    if (!skinny_gathers(M, N / 16, K)) kernel = gemm_skinny_kernel<2, true, false, SK_UNROLL, false, false>;
     if (skinny_deep(N / 16, K)) {
         if (skinny_wide_ok(W, K, ldw))
             kernel = M <= 8 ? gemm_skinny_kernel<1, true, false, SK_DEEP / 2, true>
