@@ -30,8 +30,8 @@
 //                      maximum exceeds it by 2^8 (then its O is rescaled in tensor memory), writes P as
 //                      bfloat16 over its own columns of the score buffer (tcgen05.st), and at the end
 //                      joins and normalises 64 columns of the two O and stores them.
-// Measured at the 3B sizes (24 query heads on 2 KV heads): 2,048 tokens 58 us (447 TFLOP/s; one softmax
-// in step over all 128 keys, tiles in the order of their tokens: 76), 512 tokens after 512: 18 us (27), 512
+// Measured at the 3B sizes (24 query heads on 2 KV heads): 2,048 tokens 53 us (489 TFLOP/s; one softmax
+// in step over all 128 keys, the heads one after another: 75), 512 tokens after 512: 18 us (27), 512
 // after 4,000: 48 us (65). A chunk takes 2,050 cycles; its MMAs alone would take 1,024, its 16,384
 // exponentials on the special-function units as many. What bounds it is latency: two softmax warps a scheduler
 // issue a third of the time, either unit is busy a third of the time. Handing the exponentials from half to half,
@@ -250,8 +250,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     unsigned char* v_stage = k_stage + AT_STAGES * 2 * AT_TILE;     // per stage: pages of [128 dims][page_size]
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    // a sequence's last tiles see the most keys: they start first, all heads of a tile side by side
-    const int tile = p.n_tiles - 1 - (int)(blockIdx.x / (unsigned)p.n_kv_heads);
+    // tiles start in the order of their list, which puts the ones with the most keys first, all heads of a tile side by
+    // side (2,048 tokens, us in the list's order and from its end: 24 query heads on 2 KV heads 53 and 59, 16 on 16 32 and 41)
+    const int tile = (int)(blockIdx.x / (unsigned)p.n_kv_heads);
     const int kh = (int)(blockIdx.x % (unsigned)p.n_kv_heads);
     const int seq = p.tiles[2 * tile], tok0 = p.tiles[2 * tile + 1];
     const int q_start = p.cu_q[seq];

@@ -425,14 +425,16 @@ def paged_attention(q: torch.Tensor, q_stride: int, cache: torch.Tensor, block_t
     _launched(2 if n_splits > 1 else 1)
 
 
-def attention_tile_lists(q_lens: list[int], group: int,
-                         token_tiles: bool = False) -> tuple[list[int], list[int]]:
+def attention_tile_lists(q_lens: list[int], group: int, token_tiles: bool = False,
+                         context_lens: list[int] | None = None) -> tuple[list[int], list[int]]:
     """Row tiles of the tensor-core attention for sequences that bring ``q_lens`` tokens and
     ``group`` query heads per KV head. Sequences with at most 16 rows (decode tokens) go to the
     narrow list, one (sequence, 0) tile each. The others go to the wide list: cut into 64-row
     tiles as (sequence, first row) pairs, or, with ``token_tiles`` (the tcgen05 kernel), into
     tiles of 128 // group tokens as (sequence, first token) pairs, the latest tokens first
-    because they have the most keys to walk."""
+    because they have the most keys to walk. ``context_lens`` (tokens cached before the step): these tiles go by
+    their newest position over all sequences (portions of 300, 17, 512 and 40 tokens after 0, 600, 100 and 3,000 at the
+    3B sizes: 37 us, and 44 with the sequences one after another)."""
     narrow: list[int] = []
     wide: list[int] = []
     per_tile = max(1, 128 // group)
@@ -448,6 +450,9 @@ def attention_tile_lists(q_lens: list[int], group: int,
         else:
             for row in range(0, rows, 64):
                 wide.extend((seq, row))
+    if token_tiles and context_lens is not None and wide and wide[0] != wide[-2]:
+        tiles = sorted(zip(wide[::2], wide[1::2]), key=lambda tile: -(context_lens[tile[0]] + tile[1]))
+        wide = [value for tile in tiles for value in tile]
     return narrow, wide
 
 

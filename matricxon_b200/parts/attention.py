@@ -43,7 +43,7 @@ def attention_tiles(ctx, group: int, token_tiles: bool = False):
     if cached is not None:
         return cached
     q_lens = [1] * ctx.n_seqs if ctx.padded else ctx.host.q_lens
-    narrow, wide = kernels.attention_tile_lists(q_lens, group, token_tiles)
+    narrow, wide = kernels.attention_tile_lists(q_lens, group, token_tiles, None if ctx.padded else ctx.host.context_lens)
     both = torch.tensor(narrow + wide + [0, 0], dtype=torch.int32).to(ctx.device, non_blocking=True)
     ctx.memo[key] = (both[:len(narrow)], len(narrow) // 2,
                      both[len(narrow):len(narrow) + len(wide)], len(wide) // 2)
