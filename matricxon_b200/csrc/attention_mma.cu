@@ -140,7 +140,7 @@ __device__ __forceinline__ void issue_chunk(const MmaAttnParams& p, __nv_bfloat1
                                             __nv_bfloat16* vs, unsigned long long* bar, int c0, int lo,
                                             int hi, int kept, const int* bt, const __nv_bfloat16* kbase,
                                             const __nv_bfloat16* vbase, size_t page_stride, int who,
-                                            int n_who, const int* cached = nullptr) {
+                                            int n_who) {
     const int ps = p.page_size;
     const int pages = CHUNK >> p.page_shift;
     const unsigned tile_bytes = (unsigned)(ps * HD * sizeof(__nv_bfloat16));
@@ -153,8 +153,7 @@ __device__ __forceinline__ void issue_chunk(const MmaAttnParams& p, __nv_bfloat1
             const int key0 = c0 + pg * ps;
             if (key0 <= hi && (key0 + ps - 1 >= lo || key0 < kept)) {
                 const int lp = key0 >> p.page_shift;
-                // `cached`: this chunk's block-table entries, read ahead into shared memory
-                const long long page = cached != nullptr ? cached[pg] : (lp < p.bt_stride ? bt[lp] : -1);
+                const long long page = lp < p.bt_stride ? bt[lp] : -1;
                 if (page >= 0 && page < p.n_pages) {
                     page_of[pg] = page;
                     total += 2 * tile_bytes;
@@ -185,7 +184,8 @@ __device__ __forceinline__ void issue_chunk(const MmaAttnParams& p, __nv_bfloat1
         }
 }
 
-// The same by one warp for narrow tiles, a lane a page: a decode step's attention is a chain of latencies, and one lane
+// The same by one warp for narrow tiles, a lane a page; `cached`: this chunk's block-table entries, read ahead into shared
+// memory (null: from the table). A decode step's attention is a chain of latencies, and one lane
 // that walks the pages and issues every copy took as long as the chunk's arithmetic (2,000 cycles; with this and the
 // divisions by the group taken out of a one-token tile's way, one request at 3,100 tokens of the 3B sizes decodes in
 // 1.64 instead of 1.68 ms a step). Merging the key splits as a cluster of blocks, without the kernel that follows, gained

@@ -674,8 +674,8 @@ def batched_skinny_supported(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor
 
 
 def gemm_batched_skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """``gemm_batched_simt`` without a bias for at most 16 rows of bfloat16: a warp per output column, the
-    weights read once with 16-byte loads."""
+    """``gemm_batched_simt`` without a bias for at most 16 rows of bfloat16: on the tensor cores where K is a multiple
+    of 32, a warp per output column elsewhere; the weights are read once with 16-byte loads."""
     _need(a, "a", torch.bfloat16, contiguous=False)
     _need(w, "w", torch.bfloat16)
     _need(out, "out", contiguous=False)

@@ -197,7 +197,7 @@ def batched_linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | N
         kernels.gemm_batched_skinny(x, weight, out)         # a decode step's few rows
         return out
     if x.dtype == torch.bfloat16 and bias is None and x.shape[0] > 16:
-        # more rows than the warp-per-column kernel takes (17 to 32 rows took 32 us a product on the FP32 cores at 16
+        # more rows than the kernels of a decode step take (17 to 32 rows took 32 us a product on the FP32 cores at 16
         # heads of 128 x 512): the library's strided batched product (float accumulator kept for a float result),
         # then one strided copy into the caller's interleaved layout
         if out.dtype == x.dtype and out.stride(2) == 1:
