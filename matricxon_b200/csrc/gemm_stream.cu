@@ -24,9 +24,11 @@
 //     shared memory, 39 cycles for 128 rows and 23 for 64 at 16 tokens), i.e. runs on into whatever
 //     follows in the ring. That only fills accumulator lanes that nobody reads: a row of the result
 //     depends on its own row of W.
-//   * The weights are nobody's output. Launched as a dependent of the kernel before it
-//     (programmatic dependent launch), the producer fills the whole ring with weights first and only
-//     then waits for that kernel to finish before it asks for activations.
+//   * Launched as a dependent of the kernel before it (programmatic dependent launch), the producer
+//     asks for the ring's first filling of weights towards L2 and then waits for that kernel to
+//     finish: weights may be its output like any operand (loads before the wait gained nothing: sixteen
+//     requests at the 15B sizes 1,413-1,423 us a step this way, 1,426-1,451 that way; the head in a
+//     step of 64 at the 3B sizes 2,616 and 2,608).
 // Every mbarrier wait is bounded: a wait that runs out sets MX_STATUS_WAIT_TIMEOUT and the role
 // moves on, so the block always reaches the point where tensor memory is freed.
 //
@@ -116,32 +118,20 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         const int total = n_tiles * plan.groups;
         // what a stage's loads bring: boxes of tile_rows (not rounded) weight rows and of mpad tokens
         const unsigned stage_tx = (unsigned)plan.kk * ((unsigned)plan.tile_rows * TC_BK * 2 + plan.x_slice_bytes);
-        // the ring's first filling: weights at once, activations once the kernel before this one is done
-        const int ahead = min(total, plan.stages);
-        for (int it = 0; it < ahead; ++it) {
+        // the ring's first filling of weights towards L2; loads once the kernel before this one is done
+        for (int it = 0; it < min(total, plan.stages); ++it) {
             const int tile = it / plan.groups, group = it - tile * plan.groups;
-            const int r0 = row_begin + tile * plan.tile_rows;
-            tc_mbar_expect_tx_elect(&sh.full[it], stage_tx);
-            for (int h = 0; h < plan.kk; ++h)           // columns beyond K arrive as zeros
-                tma_load_2d_elect(w_ring + (size_t)it * w_stage_bytes + (size_t)h * plan.w_slice_bytes, &map_w,
-                                  (group * plan.kk + h) * TC_BK, r0, &sh.full[it]);
+            for (int h = 0; h < plan.kk; ++h)
+                tma_prefetch_2d_elect(&map_w, (group * plan.kk + h) * TC_BK, row_begin + tile * plan.tile_rows);
         }
         pdl_wait();
-        for (int it = 0; it < ahead; ++it) {
-            const int group = it % plan.groups;
-            for (int h = 0; h < plan.kk; ++h)
-                tma_load_2d_elect(x_ring + (size_t)it * x_stage_bytes + (size_t)h * plan.x_slice_bytes, &map_x,
-                                  (group * plan.kk + h) * TC_BK, 0, &sh.full[it]);
-        }
-        bool alive = true;
-        for (int it = ahead; it < total && alive; ++it) {
+        for (int it = 0; it < total; ++it) {
             const int s = it % plan.stages;
             const int tile = it / plan.groups, group = it - tile * plan.groups;
             const int r0 = row_begin + tile * plan.tile_rows;
-            alive = tc_mbar_wait_warp(&sh.empty[s], ((unsigned)(it / plan.stages) & 1) ^ 1, status);
-            if (!alive) break;
+            if (it >= plan.stages && !tc_mbar_wait_warp(&sh.empty[s], ((unsigned)(it / plan.stages) & 1) ^ 1, status)) break;
             tc_mbar_expect_tx_elect(&sh.full[s], stage_tx);
-            for (int h = 0; h < plan.kk; ++h) {
+            for (int h = 0; h < plan.kk; ++h) {              // columns beyond K arrive as zeros
                 tma_load_2d_elect(w_ring + (size_t)s * w_stage_bytes + (size_t)h * plan.w_slice_bytes, &map_w,
                                   (group * plan.kk + h) * TC_BK, r0, &sh.full[s]);
                 tma_load_2d_elect(x_ring + (size_t)s * x_stage_bytes + (size_t)h * plan.x_slice_bytes, &map_x,

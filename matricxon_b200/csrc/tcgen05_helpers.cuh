@@ -153,6 +153,14 @@ __device__ __forceinline__ void tma_load_2d_elect(void* smem_dst, const CUtensor
         "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
 }
+// The same box towards L2 only: what a kernel may ask for before the kernel before it has ended.
+__device__ __forceinline__ void tma_prefetch_2d_elect(const CUtensorMap* map, int x, int y) {
+    asm volatile(
+        "{\n.reg .pred q;\n"
+        "elect.sync _|q, 0xffffffff;\n"
+        "@q cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];\n}\n" ::"l"(map), "r"(x), "r"(y)
+        : "memory");
+}
 // A bounded wait by a whole warp: every lane polls; the status word is set by one of them.
 __device__ __forceinline__ bool tc_mbar_wait_warp(unsigned long long* bar, unsigned parity, int* status) {
     for (int spin = 0; spin < TC_SPIN_LIMIT; ++spin)
