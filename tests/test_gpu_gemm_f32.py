@@ -40,6 +40,29 @@ def test_every_row_count_gives_the_general_kernels_bits(n, k_dim):
     assert torch.equal(few, general[:7])
 
 
+# Blocks of several weight rows, with a short last one: seven rows (1,000 columns over 148 SMs), and 17 in two rounds (4,737
+# and 5,003 columns). Pieces of six chunks of 32 (a ring filled once and one chunk more), of thirteen with a short end, of
+# twenty-four: rings that come round four times.
+@pytest.mark.parametrize("k_dim", [644, 1572, 3072])
+@pytest.mark.parametrize("n", [1000, 4737, 5003])
+def test_blocks_of_several_rows_and_rings_that_come_round(n, k_dim):
+    from matricxon_b200.ops import kernels as k
+
+    torch.manual_seed(n + k_dim)
+    a = torch.randn(130, k_dim, device=DEV)
+    w = torch.randn(n, k_dim, device=DEV) / math.sqrt(k_dim)
+    shifted = torch.empty(130 * k_dim + 1, device=DEV)[1:].view(130, k_dim).copy_(a)      # not 16-byte aligned
+    general = torch.empty(130, n, device=DEV)
+    k.gemm_simt(shifted, w, None, None, general, k.EPILOGUE_F32)
+    exact = a.double() @ w.double().T
+    bound = (k_dim / 4 + 4) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert bool(((general.double() - exact).abs() <= bound).all())
+    for m in (1, 2, 4, 8, 16, 17, 32, 33, 130):
+        out = torch.full((m, n), float("nan"), device=DEV)
+        k.gemm_simt(a[:m], w, None, None, out, k.EPILOGUE_F32)
+        assert torch.equal(out, general[:m]), m
+
+
 def test_infinities_and_nan_stay_in_their_rows():
     from matricxon_b200.ops import kernels as k
 
