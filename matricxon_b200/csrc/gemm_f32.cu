@@ -26,11 +26,14 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 
 // Decoding: the product is a stream of W from HBM. A block owns up to 32 weight rows (a lane each) and its four
 // warps take one piece of K each, so the four chains of an output are four threads. A warp keeps a ring of its own
 // of [32 rows][32 floats] of W and [rows of A][32 floats], filled by cp.async (a 128-byte line per row, chunks
-// permuted so that the 32 lanes' 16-byte reads spread over all banks): no block-wide barrier in the loop, and two
-// blocks an SM hold about 160 KB in flight. A row of A is read as a broadcast. Weights of 3072 x 12288 / 12288 x 3072 /
-// 49152 x 3072: 38 / 32 / 96 us for one row (4.0, 4.7, 6.2 TB/s), 52 / 38 / 105 us for four; the general kernel, which
-// walks tiles of 64 rows, takes 990 us for the first. From about eight rows on the reads of A from shared memory bound
-// it (128 bytes a cycle and SM go to registers, broadcast or not).
+// permuted so that the 32 lanes' 16-byte reads spread over all banks): no block-wide barrier in the loop. A row of A is
+// read as a broadcast. Weights of 3072 x 12288 / 12288 x 3072 / 49152 x 3072: 38 / 32 / 96 us for one row (4.0, 4.7, 6.2 TB/s),
+// 52 / 38 / 105 us for four; the general kernel, which walks tiles of 64 rows, takes 569 us for the first (one column of
+// K less). What is in flight bounds it: five chunks of 128 bytes a warp and weight row, so 54 KB an SM in the first (147
+// blocks of 21 rows, one an SM), 143 KB in the second while two blocks share an SM and 72 KB in its last round (439
+// blocks of 28), 159 KB in the third (31 rows); two blocks fit an SM up to four rows of A (99 to 108 KB of ring each), one
+// above. From about eight rows on the reads of A from shared memory bound it (128 bytes a cycle and SM go to registers,
+// broadcast or not): 67 us for eight in the first.
 constexpr int FR_ROWS = 32, FR_K = 32, FR_STAGES = 6, FR_THREADS = 128;
 
 template <int MB>
@@ -136,13 +139,14 @@ gemm_f32_rows_kernel(const float* __restrict__ A, int lda, const float* __restri
 // Prompts: bound by the FP32 pipes (128 multiply-adds a cycle and SM) and beside them by what shared memory hands to
 // registers, 128 bytes a cycle. A block of 128 threads forms 64 rows x 128 features of one piece of K, 8 x 8 outputs a
 // thread as 8 x 4 packed pairs of features (fma.rn.f32x2: half the issue slots). Shared memory holds a step of 16 k
-// with k outermost, so that 16 bytes of W are two pairs as the instruction wants them, and A's values twice each (the
-// other operand of a pair). The next step's operands are on their way in registers meanwhile. The four pieces of K are
+// with k outermost, so that 16 bytes of W are two pairs as the instruction wants them; the other operand, a value of A
+// twice, is formed in registers. The next step's operands are on their way in registers meanwhile. The four pieces of K are
 // the four blocks of a cluster (a 3,072-wide product of some hundred rows has too few tiles for 148 SMs otherwise);
-// each leaves its sums in its shared memory and finishes a quarter of the tile from all four. Measured at 389 rows
-// (the four products of a 3B layer): 2.28 ms, 33 TFLOP/s; unpacked from rows as they lie in memory, by cp.async, 2.38;
-// 56 rows x 256 features with 7 x 16 outputs a thread, two blocks an SM, 2.36; 64 x 192 unpacked 3.04; the general
-// kernel 4.3.
+// each leaves its sums in its shared memory and finishes a quarter of the tile from all four. 128 registers (28 bytes a
+// thread wait in local memory), four blocks an SM: issue slots 54 % and L1 74 % busy. Measured at 389 rows (the four
+// products of a 3B layer): 1.94 ms, 38 TFLOP/s; with A's values twice each in shared memory, 162 registers and three
+// blocks an SM, 2.28; unpacked from rows as they lie in memory, by cp.async, 2.38; 56 rows x 256 features with 7 x 16
+// outputs a thread, two blocks an SM, 2.36; 64 x 192 unpacked 3.04; the general kernel (a column of K less) 3.40.
 constexpr int FT_M = 64, FT_N = 128, FT_K = 16, FT_THREADS = 128;
 constexpr int FT_LDA = FT_M + 4, FT_LDW = FT_N + 4;              // floats from one k to the next
 constexpr int FT_BUFFER = FT_K * (FT_LDA + FT_LDW);

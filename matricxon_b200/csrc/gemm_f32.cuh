@@ -5,7 +5,7 @@
 
 constexpr int F32_PIECES = 4;         // chains of a sum over K: (p0 + p1) + (p2 + p3)
 // Up to here the kernel that streams the weights, in groups of 16 rows: 32 rows of the four products of a 3B layer
-// take it 0.38 ms, 33 rows take the tiles 0.60 ms.
+// take it 0.38 ms, 33 rows take the tiles 0.59 ms.
 constexpr int F32_FEW_ROWS = 32;
 
 // Length of a piece of K: a quarter, in whole steps of the kernels' loops (the last pieces may be short or empty).
