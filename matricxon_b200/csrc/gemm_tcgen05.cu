@@ -872,18 +872,18 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// A [rows, K] bfloat16 matrix with `ld` elements between rows, cut into boxes of box_rows x 64.
+// A [rows, K] matrix with `ld` elements between rows, cut into boxes of box_rows x 64 bfloat16, or of another form.
 // Encoding a map costs the host a few microseconds and a step launches some hundred products, most of
 // them on the same weight matrices and the same activation buffers as the step before: maps are kept
-// by what they describe (address, extents, row stride, box) and encoded once. A map holds no reference
+// by what they describe (address, extents, row stride, box, form) and encoded once. A map holds no reference
 // to the memory: a stale entry whose address now holds another tensor of the same extents describes
 // that tensor just as well.
 struct MapKey {
     const void* base;
     long long rows, K, ld;
-    int box_rows;
+    int box_rows, form;
     bool operator==(const MapKey& o) const {
-        return base == o.base && rows == o.rows && K == o.K && ld == o.ld && box_rows == o.box_rows;
+        return base == o.base && rows == o.rows && K == o.K && ld == o.ld && box_rows == o.box_rows && form == o.form;
     }
 };
 
@@ -899,11 +899,12 @@ std::mutex g_map_cache_lock;
 
 }  // namespace
 
-int mx_tensor_map_2d(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows) {
-    const MapKey key = {base, rows, K, ld, box_rows};
+int mx_tensor_map_form(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows,
+                       int form) {
+    const MapKey key = {base, rows, K, ld, box_rows, form};
     unsigned long long h = (unsigned long long)(size_t)base * 0x9E3779B97F4A7C15ull;
     h ^= (unsigned long long)rows * 0xC2B2AE3D27D4EB4Full + (unsigned long long)K * 0x165667B19E3779F9ull +
-         (unsigned long long)ld * 0x27D4EB2F165667C5ull + (unsigned long long)box_rows;
+         (unsigned long long)ld * 0x27D4EB2F165667C5ull + (unsigned long long)(box_rows + 512 * form);
     h ^= h >> 29;
     std::lock_guard<std::mutex> guard(g_map_cache_lock);
     MapSlot& slot = g_map_cache[h & (MAP_CACHE_SLOTS - 1)];
@@ -914,17 +915,23 @@ int mx_tensor_map_2d(CUtensorMap* map, const void* base, long long rows, long lo
     EncodeTiledFn encode = encode_tiled_fn();
     if (encode == nullptr) MX_REFUSE("tcgen05 gemm: the driver does not offer cuTensorMapEncodeTiled");
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows};
+    const bool f32 = form == MX_MAP_F32_128B, narrow = form == MX_MAP_BF16_64B;
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * (f32 ? 4 : 2)};
+    const cuuint32_t box[2] = {(cuuint32_t)(f32 || narrow ? 32 : TC_BK), (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
-    const CUresult rc = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,
-                               box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+    const CUresult rc = encode(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                               const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                               narrow ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (rc != CUDA_SUCCESS) MX_REFUSE("tcgen05 gemm: cuTensorMapEncodeTiled failed with code %d", (int)rc);
     slot.key = key;
     slot.map = *map;
     slot.used = true;
     return MX_OK;
+}
+
+int mx_tensor_map_2d(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows) {
+    return mx_tensor_map_form(map, base, rows, K, ld, box_rows, MX_MAP_BF16_128B);
 }
 
 namespace {

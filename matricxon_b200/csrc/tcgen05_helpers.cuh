@@ -10,6 +10,11 @@
 // A [rows, K] bfloat16 matrix with `ld` elements between rows, cut into boxes of box_rows x 64
 // (128-byte swizzle). Encoded once per distinct operand and kept (gemm_tcgen05.cu).
 int mx_tensor_map_2d(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows);
+// The same in another form: boxes of 64 or 32 bfloat16 or of 32 floats, in rows of 128 or 64 bytes swizzled over as many.
+#define MX_MAP_BF16_128B 0
+#define MX_MAP_F32_128B 1
+#define MX_MAP_BF16_64B 2
+int mx_tensor_map_form(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows, int form);
 
 namespace {
 

@@ -202,6 +202,46 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None,
     _launched()
 
 
+def split_gemm_supported(a: torch.Tensor, w: torch.Tensor) -> bool:
+    return (a.dtype == torch.float32 and w.dtype == torch.float32 and a.shape[1] % 4 == 0 and a.stride(1) == 1
+            and a.stride(0) % 4 == 0 and w.is_contiguous() and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def split_gemm_pays(m: int, n: int, k: int) -> bool:
+    """Whether a float product that the split kernel takes is better off there than on the FP32 cores
+    (gemm_f32_split.cu)."""
+    return bool(library().mx_gemm_f32_split_pays(m, n, k))
+
+
+def gemm_f32_split(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None,
+                   residual: torch.Tensor | None, out: torch.Tensor, mode: int,
+                   status: torch.Tensor | None = None) -> None:
+    """The float product on the tcgen05 tensor cores: every float as the sum of three bfloat16 numbers, six products
+    of them, sums rounded to nearest every 32 values of K (no less exact than the FP32 cores' sums)."""
+    _need(a, "a", torch.float32, contiguous=False)
+    _need(w, "w", torch.float32)
+    _need(out, "out", torch.float32)
+    if a.stride(1) != 1:
+        raise KernelLibraryError("a must have unit stride along K")
+    m, k = a.shape
+    n = w.shape[0]
+    assert w.shape[1] == k and tuple(out.shape) == (m, n), (a.shape, w.shape, out.shape)
+    if bias is not None:
+        _need(bias, "bias", torch.float32)
+        assert bias.numel() == n
+    if residual is not None:
+        _need(residual, "residual", torch.float32)
+        assert tuple(residual.shape) == (m, n) and residual.stride(0) == out.stride(0)
+    if status is None:
+        status = default_status(a.device)
+    need = library().mx_gemm_f32_split_scratch(m, n, k)
+    scratch = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
+    check(library().mx_gemm_f32_split(_ptr(a), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), _ptr(scratch), m, n, k,
+                                      a.stride(0), w.stride(0), out.stride(0), mode, _ptr(status), _stream()),
+          "gemm_f32_split")
+    _launched()
+
+
 _default_status: dict[int, torch.Tensor] = {}
 
 

@@ -36,6 +36,9 @@ _SIGNATURES: dict[str, tuple[list, object]] = {
     "mx_epilogue": ([P, I, P, P, P, I, L, I, I, P], I),
     "mx_gemm_simt": ([P, P, I, P, P, P, I, I, I, I, I, I, I, I, P], I),
     "mx_gemm_f32_pays": ([I, I, I], I),
+    "mx_gemm_f32_split_pays": ([I, I, I], I),
+    "mx_gemm_f32_split_scratch": ([I, I, I], L),
+    "mx_gemm_f32_split": ([P, P, P, P, P, P, I, I, I, I, I, I, I, P, P], I),
     "mx_gemm_tcgen05": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P, P], I),
     "mx_gemm_tcgen05_force_tiles": ([I], I),
     "mx_gemm_stream_pays": ([I, I, I], I),

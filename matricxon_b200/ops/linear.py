@@ -1,7 +1,8 @@
 """``out = epilogue(x @ W.T + bias)``: the one matrix product every part uses.
 
 Backends, chosen by the runtime:
-  "simt"    -- the engine's own FP32-core kernel; the only backend of the 32-bit path.
+  "simt"    -- the engine's own FP32-core kernels.
+  "split"   -- the engine's tcgen05 kernel of the 32-bit path: each float as three bfloat16 numbers.
   "skinny"  -- the engine's tensor-core kernel for at most 16 rows (decoding): the weight
                matrix is streamed once and the epilogue is fused.
   "stream"  -- the engine's TMA + tcgen05 kernel for at most 128 rows with the tokens as the
@@ -11,7 +12,7 @@ Backends, chosen by the runtime:
   "library" -- cuBLAS through ``torch.mm`` for bfloat16 (the reference runs its products
                through nn.Linear, i.e. the library: app/architectures/qwen_layers.py:50-53),
                followed by the engine's fused bias / GELU / residual epilogue kernel.
-  "auto"    -- "simt" for float32; for bfloat16 "skinny" up to 16 rows, "tcgen05" above 256 rows,
+  "auto"    -- for float32 "split" where it pays, else "simt"; for bfloat16 "skinny" up to 16 rows, "tcgen05" above 256 rows,
                "library" between (a weight stream that 128-row tiles would leave to a few SMs) and
                for shapes neither takes (a K that is no multiple of 8), and "stream" from 9 rows
                on for large matrices (``_pick`` gives the measured thresholds).
@@ -52,8 +53,8 @@ def resolve_backend(requested: str, dtype: torch.dtype) -> str:
     if dtype == torch.float32:
         if requested not in ("auto", "simt"):
             raise KernelLibraryError(
-                f"the float32 path runs on the FP32-core kernel only, not {requested!r}")
-        return "simt"
+                f"the float32 path runs on the engine's float kernels only, not {requested!r}")
+        return requested
     if requested not in ("auto", "simt", "skinny", "stream", "tcgen05", "library"):
         raise KernelLibraryError(f"unknown GEMM backend {requested!r}")
     return requested
@@ -68,6 +69,9 @@ def _pick(x: torch.Tensor, weight: torch.Tensor, m: int, n: int) -> str:
     requests decoding at the 3B sizes 2.40 -> 2.12 ms a step against a limit of 64 weight rows per SM). For 17 to 128 rows
     it wins where every SM owns 256 weight rows (the head: 59 against 66 us for the library's product plus the epilogue
     kernel)."""
+    if x.dtype == torch.float32:
+        pays = kernels.split_gemm_pays(m, n, x.shape[1]) and kernels.split_gemm_supported(x, weight)
+        return "split" if pays else "simt"
     if 9 <= m <= 128 and kernels.stream_gemm_supported(x, weight):
         sms = kernels.sm_count(x.device)
         if kernels.stream_gemm_pays(n, x.shape[1], sms) if m <= 16 else -(-n // sms) >= 256:
@@ -161,6 +165,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, mod
         return out
     if backend == "simt":
         kernels.gemm_simt(x, weight, bias, residual, out, mode)
+        return out
+    if backend == "split":
+        kernels.gemm_f32_split(x, weight, bias, residual, out, mode)
         return out
     if backend == "skinny":
         kernels.gemm_skinny(x, weight, bias, residual, out, mode)

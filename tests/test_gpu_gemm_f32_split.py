@@ -1,0 +1,88 @@
+"""Float products on the tensor cores, three bfloat16 numbers a float: against 64 bits at the edges of tiles, stages and
+shares of K, no further off than the FP32 cores, every epilogue, and what is not finite."""
+
+import math
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a GPU")]
+DEV = "cuda:0"
+
+
+# tokens: a tile of 16, one row more, the last that are split in passing and one more, a tile of 208 and one more, several
+# tiles; columns: less than a tile, ragged, several tiles; K: less than a stage, ragged stages, shares of K of 5 and 6 stages
+@pytest.mark.parametrize("m", [1, 16, 17, 64, 65, 130, 208, 209, 700])
+@pytest.mark.parametrize("n,k_dim", [(1, 4), (131, 36), (260, 332), (1027, 1500), (384, 3072)])
+def test_against_64_bits_and_the_fp32_cores(m, n, k_dim):
+    from matricxon_b200.ops import kernels as k
+
+    torch.manual_seed(m * 1000 + n)
+    a = torch.randn(m, k_dim + 4, device=DEV)[:, :k_dim]                   # rows of a wider buffer
+    w = torch.randn(n, k_dim, device=DEV) / math.sqrt(k_dim)
+    bias, residual = torch.randn(n, device=DEV), torch.randn(m, n, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    exact = a.double() @ w.double().T
+    out, plain = torch.full((m, n), float("nan"), device=DEV), torch.empty(m, n, device=DEV)
+    k.gemm_f32_split(a, w, None, None, out, k.EPILOGUE_F32, status)
+    k.gemm_simt(a, w, None, None, plain, k.EPILOGUE_F32)
+    # each 32 values of k: the parts left out (2^-26 of a term), twelve cut-offs of a sum below |a| . |w|, one rounding
+    size = a.double().abs() @ w.double().abs().T
+    assert bool(((out.double() - exact).abs() <= (2.0 ** -25 + 13 * 2.0 ** -23) * size).all())
+    if m * n > 4000 and k_dim > 300:
+        assert (out.double() - exact).norm() <= (plain.double() - exact).norm()
+    # the epilogues add to the same sums
+    biased = torch.empty_like(out)
+    k.gemm_f32_split(a, w, bias, residual, biased, k.EPILOGUE_RESIDUAL, status)
+    assert torch.equal(biased, residual + (out + bias))
+    inplace = residual.clone()
+    k.gemm_f32_split(a, w, bias, inplace, inplace, k.EPILOGUE_RESIDUAL, status)
+    assert torch.equal(inplace, biased)
+    k.gemm_f32_split(a, w, bias, None, biased, k.EPILOGUE_GELU, status)
+    ref = torch.nn.functional.gelu((out + bias).double(), approximate="tanh")
+    assert bool(((biased.double() - ref).abs() <= 2e-6 * (1 + ref.abs())).all())
+    assert status.item() == 0
+
+
+def test_sizes_of_numbers():
+    """Rows of very large, very small and subnormal floats, and terms that cancel."""
+    from matricxon_b200.ops import kernels as k
+
+    a, w = torch.randn(40, 256, device=DEV), torch.randn(300, 256, device=DEV)
+    scale = torch.tensor([2.0 ** e for e in (-120, -60, 0, 60, 100)], device=DEV).repeat(8)[:, None]
+    out, plain = torch.empty(40, 300, device=DEV), torch.empty(40, 300, device=DEV)
+    k.gemm_f32_split(a, w, None, None, out, k.EPILOGUE_F32)
+    k.gemm_f32_split(a * scale, w, None, None, plain, k.EPILOGUE_F32)
+    big = scale[:, 0] > 2.0 ** -100
+    assert torch.equal(plain[big], (out * scale)[big])                     # powers of two move exponents only
+    # third parts of 2^-120 are below the smallest subnormal (2^-133): up to that of each term is lost
+    assert bool(((plain[~big].double() - (out * scale)[~big].double()).abs() <= 256 * 5 * 2.0 ** -133).all())
+    twice = torch.cat([a, -a], dim=1).contiguous()
+    k.gemm_f32_split(twice, torch.cat([w, w], dim=1).contiguous(), None, None, out, k.EPILOGUE_F32)
+    size = 2 * (a.double().abs() @ w.double().abs().T)
+    assert bool((out.double().abs() <= (2.0 ** -25 + 13 * 2.0 ** -23) * size).all())
+
+
+def test_infinities_and_nan_stay_in_their_rows():
+    from matricxon_b200.ops import kernels as k
+
+    for m in (20, 300):
+        a, w = torch.randn(m, 512, device=DEV), torch.randn(261, 512, device=DEV)
+        a[0, 5], a[1, 511], a[2, 3] = math.inf, math.nan, 3.4e38           # the last rounds to infinity in bfloat16
+        w[7, 3] = 0.5
+        out, plain = torch.empty(m, 261, device=DEV), torch.empty(m, 261, device=DEV)
+        k.gemm_f32_split(a, w, None, None, out, k.EPILOGUE_F32)
+        k.gemm_simt(a, w, None, None, plain, k.EPILOGUE_F32)
+        assert torch.equal(out[0], w[:, 5].sign() * math.inf) and bool(out[1].isnan().all())
+        assert torch.equal(out[2], plain[2]) and bool(out[2, 7].isfinite())
+        assert bool(out[3:].isfinite().all())
+
+
+def test_the_engine_takes_it_for_many_rows():
+    from matricxon_b200.ops.linear import chosen_backend
+
+    w = torch.empty(512, 512, device=DEV)
+    assert chosen_backend(torch.empty(200, 512, device=DEV), w) == "split"
+    assert chosen_backend(torch.empty(200, 512, device=DEV), w, "simt") == "simt"
+    assert chosen_backend(torch.empty(200, 513, device=DEV)[:, 1:], w) == "simt"      # cannot be read 16 bytes at a time
