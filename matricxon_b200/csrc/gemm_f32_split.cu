@@ -510,8 +510,14 @@ FsPlan fs_plan(int M, int N, int K) {
 
 }  // namespace
 
-// Whether a float product is better off here than on the FP32 cores (gemm_f32.cu).
-extern "C" int mx_gemm_f32_split_pays(int M, int N, int K) { return M > 16 && N >= 256 && K >= 256; }
+// Whether a float product is better off here than on the FP32 cores (gemm_f32.cu): K long enough for what a tile costs
+// beside its stages (some 9 us with the launch). Us there against here: 17 rows x 256 x 256 6.7 and 9.4, 17 x 4,096 x 512
+// 10.6 and 13.1, 33 x 4,096 x 512 16.9 and 13.5, 17 x 1,024 x 1,024 17.2 and 12.7, 512 x 256 x 256 11.4 and 15.1, 512 x 512 x
+// 512 16.4 and 15.8; 16 rows x 4,096 x 512 6.1 and 11.6, 9 x 2,048 x 2,048 16.5 and 15.5, 16 x 3,072 x 12,288 82 and 52; 4 rows
+// x 3,072 x 12,288 50 and 51.
+extern "C" int mx_gemm_f32_split_pays(int M, int N, int K) {
+    return N >= 256 && K >= (M > 32 ? 512 : M > 16 ? 1024 : 2048) && M > 8;
+}
 
 // Bytes of scratch that a product needs (0: none): the parts of A where a tile has more tokens than are split in passing.
 extern "C" long long mx_gemm_f32_split_scratch(int M, int N, int K) {
