@@ -308,6 +308,205 @@ paged_attention_kernel(const AttnParams p) {
     }
 }
 
+// ---- float, heads of 128 numbers, pages of whole sixteens: a warp per sixteen keys ---------------------------------
+// The kernel above stages keys and values in shared memory for a block, 32 keys at a time between barriers: two or three
+// trips to memory one after another and value writes of eight to a bank. Here a warp owns sixteen keys (a run inside one
+// page) for the token's heads of one KV head, and what it loads goes straight to registers: a key's row is 512 bytes side
+// by side (four numbers a lane; scores are summed over the lanes by halving, sixteen keys at once), and a lane takes four
+// value dimensions of sixteen slots, 64 bytes each. The four warps of a block walk the chunks of its share in turn, each
+// with a softmax of its own, and are combined at the end. Bound by the multiply-adds of long prompts (two thirds of the
+// instructions) and by one trip to memory in decoding.
+constexpr int F32A_KEYS = 16, F32A_DIM = 128;
+
+__device__ __forceinline__ void load8(const float* p, float* v) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p));
+}
+
+// HEADS: query heads of a block, padded.
+template <int HEADS>
+__global__ void __launch_bounds__(ATT_THREADS)
+paged_attention_f32_kernel(const AttnParams p) {
+    __shared__ float4 weights[ATT_WARPS][HEADS][F32A_KEYS / 4];
+    __shared__ float sums[ATT_WARPS][HEADS][F32A_DIM];
+    __shared__ float maxima[ATT_WARPS][HEADS], totals[ATT_WARPS][HEADS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = blockIdx.x, split = blockIdx.z;
+    const int group = p.n_heads / p.n_kv_heads, n_hgroups = (group + HEADS - 1) / HEADS;
+    const int kh = blockIdx.y / n_hgroups, hg = blockIdx.y - kh * n_hgroups;
+    const int head0 = kh * group + hg * HEADS, heads = min(HEADS, group - hg * HEADS);
+
+    pdl_trigger();
+    pdl_wait();
+    const float* q = after_wait(reinterpret_cast<const float*>(p.q));
+    const float* cache = after_wait(reinterpret_cast<const float*>(p.cache));
+    const int seq = p.tok_seq[t];
+    if (seq < 0) {  // a padding row of a fixed-size batch: defined output, no cache access
+        for (int h = 0; h < heads; ++h) {
+            const int d = threadIdx.x;
+            if (split == 0) reinterpret_cast<float*>(p.out)[(size_t)t * p.out_stride + (size_t)(head0 + h) * F32A_DIM + d] = 0.f;
+            if (p.n_splits > 1) {
+                const size_t base = ((size_t)t * p.n_heads + head0 + h) * p.n_splits + split;
+                p.part_o[base * F32A_DIM + d] = 0.f;
+                if (d == 0) { p.part_ml[base * 2] = 0.f; p.part_ml[base * 2 + 1] = 1.f; }
+            }
+        }
+        return;
+    }
+    const int pos = p.positions[t], hi = pos, lo = first_visible_key(pos, p.window);
+    // the walk over chunks, kept keys first, as in the kernel above
+    const int kept = lo > 0 ? min(p.keep_first, lo) : 0;
+    const int first_chunk = lo / F32A_KEYS, last_chunk = hi / F32A_KEYS;
+    const int n_kept = min((kept + F32A_KEYS - 1) / F32A_KEYS, first_chunk);
+    const int n_chunks = n_kept + last_chunk - first_chunk + 1;
+    const int per_split = (n_chunks + p.n_splits - 1) / p.n_splits;
+    const int c_begin = split * per_split, c_end = min(n_chunks, c_begin + per_split);
+    const int* bt = p.block_tables + (size_t)seq * p.bt_stride;
+    const size_t head_stride = (size_t)p.page_size * F32A_DIM;
+
+    float4 qv[HEADS];
+    float acc[HEADS][4], m_run[HEADS], l_run[HEADS];                       // l_run: of this lane's keys
+#pragma unroll
+    for (int h = 0; h < HEADS; ++h) {
+        qv[h] = h < heads ? reinterpret_cast<const float4*>(q + (size_t)t * p.q_stride + (size_t)(head0 + h) * F32A_DIM)[lane]
+                          : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[h][i] = 0.f;
+        m_run[h] = -INFINITY;
+        l_run[h] = 0.f;
+    }
+    for (int c = c_begin + warp; c < c_end; c += ATT_WARPS) {
+        const int c0 = (c < n_kept ? c : first_chunk + c - n_kept) * F32A_KEYS;
+        const int lp = c0 / p.page_size, off = c0 - lp * p.page_size;
+        long long page = lp < p.bt_stride ? bt[lp] : -1;
+        const bool there = page >= 0 && page < p.n_pages;
+        if (!there) {                                   // keys that no page holds read as zeros
+            if (lane == 0) atomicOr(p.status, MX_STATUS_BAD_PAGE);
+            page = 0;
+        }
+        const float* keys = cache + ((size_t)page * 2 * p.n_kv_heads + kh) * head_stride + (size_t)off * F32A_DIM;
+        const float* values = cache + ((size_t)page * 2 * p.n_kv_heads + p.n_kv_heads + kh) * head_stride + off;
+        float4 kv[F32A_KEYS];
+#pragma unroll
+        for (int j = 0; j < F32A_KEYS; ++j) {
+            kv[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (there && c0 + j <= hi) kv[j] = reinterpret_cast<const float4*>(keys + (size_t)j * F32A_DIM)[lane];
+        }
+        // a lane ends with the score of key lane / 2
+        const int kpos = c0 + (lane >> 1);
+        const bool valid = (kpos >= lo || kpos < kept) && kpos <= hi;
+        float score[HEADS];
+#pragma unroll
+        for (int h = 0; h < HEADS; ++h) {
+            float s[F32A_KEYS];
+#pragma unroll
+            for (int j = 0; j < F32A_KEYS; ++j)
+                s[j] = fmaf(qv[h].w, kv[j].w, fmaf(qv[h].z, kv[j].z, fmaf(qv[h].y, kv[j].y, qv[h].x * kv[j].x)));
+#pragma unroll
+            for (int half = F32A_KEYS / 2; half > 0; half >>= 1) {
+                const bool upper = lane & (2 * half);
+#pragma unroll
+                for (int j = 0; j < half; ++j) {
+                    const float give = upper ? s[j] : s[j + half], keep = upper ? s[j + half] : s[j];
+                    s[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * half);
+                }
+            }
+            score[h] = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);
+        }
+        float v[4][F32A_KEYS] = {};                     // dimension lane + 32 i, on its way during the softmax
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float* from = values + (size_t)(lane + 32 * i) * p.page_size;
+            if (there) {
+                load8(from, v[i]);
+                load8(from + 8, v[i] + 8);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < HEADS; ++h) {
+            float sv = score[h] * p.scale;
+            if (p.softcap > 0.f) sv = p.softcap * tanhf(sv / p.softcap);
+            if (p.distance && valid && h < heads)
+                sv -= p.distance[head0 + h] * logf(fmaf(p.distance[p.n_heads + head0 + h], (float)(pos - kpos), 1.f));
+            sv = valid ? sv : -INFINITY;
+            const float m_new = fmaxf(m_run[h], warp_max(sv));
+            const float pj = valid ? expf(sv - m_new) : 0.f;
+            const float alpha = m_run[h] == -INFINITY ? 0.f : expf(m_run[h] - m_new);
+            l_run[h] = l_run[h] * alpha + pj;
+            m_run[h] = m_new;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[h][i] *= alpha;
+            if ((lane & 1) == 0) reinterpret_cast<float*>(weights[warp][h])[lane >> 1] = pj;
+        }
+        if (!there || c0 < lo || c0 + F32A_KEYS - 1 > hi) {
+            // slots that are out of sight may hold anything
+#pragma unroll
+            for (int j = 0; j < F32A_KEYS; ++j) {
+                const bool seen = there && (c0 + j >= lo || c0 + j < kept) && c0 + j <= hi;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i][j] = seen ? v[i][j] : 0.f;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < HEADS; ++h) {
+#pragma unroll
+            for (int j = 0; j < F32A_KEYS / 4; ++j) {
+                const float4 w = weights[warp][h][j];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    acc[h][i] = fmaf(w.x, v[i][4 * j], acc[h][i]);
+                    acc[h][i] = fmaf(w.y, v[i][4 * j + 1], acc[h][i]);
+                    acc[h][i] = fmaf(w.z, v[i][4 * j + 2], acc[h][i]);
+                    acc[h][i] = fmaf(w.w, v[i][4 * j + 3], acc[h][i]);
+                }
+            }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int h = 0; h < HEADS; ++h) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sums[warp][h][lane + 32 * i] = acc[h][i];
+        const float total = 0.5f * warp_sum(l_run[h]);                     // every key stands in two lanes
+        if (lane == 0) { maxima[warp][h] = m_run[h]; totals[warp][h] = total; }
+    }
+    __syncthreads();
+    const int d = threadIdx.x;
+    for (int h = 0; h < heads; ++h) {
+        float m = -INFINITY, l = 0.f, o = 0.f;
+#pragma unroll
+        for (int w = 0; w < ATT_WARPS; ++w) m = fmaxf(m, maxima[w][h]);
+#pragma unroll
+        for (int w = 0; w < ATT_WARPS; ++w) {
+            const float factor = maxima[w][h] == -INFINITY ? 0.f : expf(maxima[w][h] - m);
+            l += totals[w][h] * factor;
+            o += sums[w][h][d] * factor;
+        }
+        if (p.n_splits == 1) {
+            if (p.sink) l += expf(p.sink[head0 + h] - m);
+            reinterpret_cast<float*>(p.out)[(size_t)t * p.out_stride + (size_t)(head0 + h) * F32A_DIM + d] = o / l;
+        } else {
+            const size_t base = ((size_t)t * p.n_heads + head0 + h) * p.n_splits + split;
+            p.part_o[base * F32A_DIM + d] = o;
+            if (d == 0) { p.part_ml[base * 2] = m; p.part_ml[base * 2 + 1] = l; }
+        }
+    }
+}
+
+template <int HEADS>
+int launch_attention_f32(const AttnParams& p, int n_tokens, cudaStream_t stream) {
+    const int group = p.n_heads / p.n_kv_heads;
+    const dim3 grid(n_tokens, p.n_kv_heads * ((group + HEADS - 1) / HEADS), p.n_splits);
+    const cudaError_t e = mx_launch_chained(paged_attention_f32_kernel<HEADS>, grid, dim3(ATT_THREADS), 0, stream, p);
+    if (e != cudaSuccess) {
+        mx_set_error("attention: launch failed: %s", cudaGetErrorString(e));
+        return (int)e;
+    }
+    return MX_OK;
+}
+
 template <typename T>
 __global__ void attention_merge_kernel(const float* __restrict__ part_o,
                                        const float* __restrict__ part_ml, T* __restrict__ out,
@@ -462,6 +661,13 @@ size_t attention_smem_bytes(int head_dim) {
            2 * (size_t)KEYS * head_dim * sizeof(T);
 }
 
+// Whether the float kernel takes a call: its loads are 16 bytes of a query and 32 of a value row.
+template <typename T>
+bool sixteen_keys_a_warp(const AttnParams& p) {
+    return sizeof(T) == 4 && p.head_dim == F32A_DIM && p.page_size % F32A_KEYS == 0 && p.q_stride % 4 == 0 &&
+           (reinterpret_cast<uintptr_t>(p.q) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.cache) & 31) == 0;
+}
+
 template <typename T, int HD_SLOTS>
 int launch_attention(const AttnParams& p, int n_tokens, cudaStream_t stream) {
     const size_t smem = attention_smem_bytes<T>(p.head_dim);
@@ -473,8 +679,16 @@ int launch_attention(const AttnParams& p, int n_tokens, cudaStream_t stream) {
     const int group = p.n_heads / p.n_kv_heads;
     const int n_hgroups = (group + GH - 1) / GH;
     dim3 grid(n_tokens, p.n_kv_heads * n_hgroups, p.n_splits);
-    paged_attention_kernel<T, HD_SLOTS><<<grid, ATT_THREADS, smem, stream>>>(p);
-    int rc = mx_launch_status();
+    int rc;
+    if (sixteen_keys_a_warp<T>(p)) {
+        const int parts = (group + 11) / 12, heads = (group + parts - 1) / parts;       // of a block, evenly dealt
+        rc = heads <= 4 ? launch_attention_f32<4>(p, n_tokens, stream)
+             : heads <= 8 ? launch_attention_f32<8>(p, n_tokens, stream)
+                          : launch_attention_f32<12>(p, n_tokens, stream);
+    } else {
+        paged_attention_kernel<T, HD_SLOTS><<<grid, ATT_THREADS, smem, stream>>>(p);
+        rc = mx_launch_status();
+    }
     if (rc != MX_OK || p.n_splits == 1) return rc;
     return launch_merge<T>(p.part_o, p.part_ml, (T*)p.out, p.out_stride, n_tokens, p.n_heads, p.head_dim, p.n_splits,
                            p.sink, stream);
