@@ -433,6 +433,112 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     }
 }
 
+// ------------------------------------------------------------------------------------------- up to eight rows
+// Decoding: a stream of the weights. A block of eight warps owns 16 weight rows, the rows of mma.sync.m16n8k16, with the
+// tokens as its columns; the warps deal out K, 32 values at a time. A lane loads floats of two weight rows (64 bytes of a
+// row to a quad) and of a token, splits them where they are and multiplies: nothing passes through shared memory. Three
+// pieces are in flight a warp, two blocks an SM.
+constexpr int FK_WARPS = 8, FK_THREADS = 32 * FK_WARPS, FK_ROWS = 16, FK_TOKENS = 8, FK_UNROLL = 3;
+
+__device__ __forceinline__ void mma_parts(float (&d)[4], const unsigned (&a)[2][4], const unsigned (&b)[4], int j) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0][2 * j]), "r"(a[1][2 * j]), "r"(a[0][2 * j + 1]), "r"(a[1][2 * j + 1]), "r"(b[2 * j]), "r"(b[2 * j + 1]));
+}
+
+__device__ __forceinline__ float4 load_once(const float* p) {
+    float4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
+__global__ void __launch_bounds__(FK_THREADS, 2)
+gemm_f32_skinny_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw,
+                       const float* __restrict__ bias, const float* residual, float* out, int ldo, int M, int N, int K,
+                       int mode) {
+    __shared__ float sums[FK_WARPS][FK_TOKENS][FK_ROWS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int n0 = blockIdx.x * FK_ROWS, pieces = (K + 31) / 32;
+    const float* w_row[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) w_row[i] = W + (size_t)min(n0 + g + 8 * i, N - 1) * ldw;
+    // the weights' first lines set out for L2 while the kernel before this one ends
+    for (int u = 0; u < FK_UNROLL; ++u) {
+        const int k = 32 * (warp + FK_WARPS * u);
+        if (t == 0 && k < K) {
+            prefetch_l2(w_row[0] + k);
+            prefetch_l2(w_row[1] + k);
+        }
+    }
+    pdl_wait();
+    A = after_wait(A);
+    W = after_wait(W);
+    bias = after_wait(bias);
+    const float* x_row = A + (size_t)min(g, M - 1) * lda;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) w_row[i] = after_wait(w_row[i]);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int first = warp; first < pieces; first += FK_WARPS * FK_UNROLL) {
+        float4 w[FK_UNROLL][2][2], x[FK_UNROLL][2];
+#pragma unroll
+        for (int u = 0; u < FK_UNROLL; ++u)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int k = 32 * (first + FK_WARPS * u) + 16 * e + 4 * t;              // K is a multiple of 4
+                const bool in = k < K;
+                const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+                w[u][0][e] = in ? load_once(w_row[0] + k) : none;
+                w[u][1][e] = in ? load_once(w_row[1] + k) : none;
+                x[u][e] = in ? *reinterpret_cast<const float4*>(x_row + k) : none;
+            }
+#pragma unroll
+        for (int u = 0; u < FK_UNROLL; ++u) {
+            unsigned wh[2][4], wm[2][4], wl[2][4], xh[4], xm[4], xl[4];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    split_pair(w[u][i][e].x, w[u][i][e].y, wh[i][2 * e], wm[i][2 * e], wl[i][2 * e]);
+                    split_pair(w[u][i][e].z, w[u][i][e].w, wh[i][2 * e + 1], wm[i][2 * e + 1], wl[i][2 * e + 1]);
+                }
+                split_pair(x[u][e].x, x[u][e].y, xh[2 * e], xm[2 * e], xl[2 * e]);
+                split_pair(x[u][e].z, x[u][e].w, xh[2 * e + 1], xm[2 * e + 1], xl[2 * e + 1]);
+            }
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                mma_parts(c, wl, xh, j);
+                mma_parts(c, wh, xl, j);
+                mma_parts(c, wm, xm, j);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                mma_parts(c, wm, xh, j);
+                mma_parts(c, wh, xm, j);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) mma_parts(c, wh, xh, j);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i] += c[i];
+        }
+    }
+    pdl_trigger();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sums[warp][2 * t + (i & 1)][g + 8 * (i >> 1)] = acc[i];
+    __syncthreads();
+    const int f = threadIdx.x % FK_ROWS, m = threadIdx.x / FK_ROWS, n = n0 + f;
+    if (m >= M || m >= FK_TOKENS || n >= N) return;
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < FK_WARPS; ++w) v += sums[w][m][f];
+    if (!isfinite(v)) v = plain_product(A + (size_t)m * lda, W + (size_t)n * ldw, K);
+    v = mode_activation(v + (bias != nullptr ? bias[n] : 0.f), mode);
+    const size_t o = (size_t)m * ldo + n;
+    if (mode == MX_MODE_RESIDUAL) v += residual[o];
+    out[o] = v;
+}
+
 // ------------------------------------------------------------------------------------------- the host's side
 constexpr int FS_MAX_SPLITS = 8;
 
@@ -515,8 +621,13 @@ FsPlan fs_plan(int M, int N, int K) {
 // 10.6 and 13.1, 33 x 4,096 x 512 16.9 and 13.5, 17 x 1,024 x 1,024 17.2 and 12.7, 512 x 256 x 256 11.4 and 15.1, 512 x 512 x
 // 512 16.4 and 15.8; 16 rows x 4,096 x 512 6.1 and 11.6, 9 x 2,048 x 2,048 16.5 and 15.5, 16 x 3,072 x 12,288 82 and 52; 4 rows
 // x 3,072 x 12,288 50 and 51.
+// Up to eight rows, on the kernel for them: 4 rows x 3,072 x 12,288 50 and 40, 4 x 12,288 x 3,072 36 and 33, 8 x 12,288 x
+// 3,072 52 and 33, 4 x 1,024 x 1,024 6.0 and 5.2; but 4 x 49,152 x 3,072 103 and 110, 4 x 4,096 x 512 4.2 and 4.7, and one or
+// two rows 5 to 15 % slower everywhere (2 x 12,288 x 3,072 31.6 and 32.1).
 extern "C" int mx_gemm_f32_split_pays(int M, int N, int K) {
-    return N >= 256 && K >= (M > 32 ? 512 : M > 16 ? 1024 : 2048) && M > 8;
+    if (N < 256 || M <= 2) return 0;
+    if (M <= 4) return K >= 1024 && N <= 16384;
+    return K >= (M <= 8 ? 512 : M <= 16 ? 2048 : M <= 32 ? 1024 : 512);
 }
 
 // Bytes of scratch that a product needs (0: none): the parts of A where a tile has more tokens than are split in passing.
@@ -539,6 +650,15 @@ extern "C" int mx_gemm_f32_split(const float* A, const float* W, const float* bi
     if (status == nullptr) MX_REFUSE("split gemm: a status word is needed for its bounded waits");
     if (3LL * M > 0x7fffffffLL) MX_REFUSE("split gemm: M = %d is beyond this kernel's coordinates", M);
 
+    if (M <= FK_TOKENS) {
+        const cudaError_t e = mx_launch_chained(gemm_f32_skinny_kernel, dim3((N + FK_ROWS - 1) / FK_ROWS), dim3(FK_THREADS), 0,
+                                                stream, A, lda, W, ldw, bias, residual, out, ldo, M, N, K, mode);
+        if (e != cudaSuccess) {
+            mx_set_error("split gemm: launch failed: %s", cudaGetErrorString(e));
+            return (int)e;
+        }
+        return MX_OK;
+    }
     static bool attribute_set = false;
     if (!attribute_set) {
         if (cudaFuncSetAttribute(gemm_f32_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FS_SMEM) != cudaSuccess)
