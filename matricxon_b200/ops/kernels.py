@@ -290,6 +290,36 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None,
     _launched()
 
 
+def columns_gemm_pays(m: int, n: int, k: int) -> bool:
+    """Whether a product of more than 256 rows is better off with its tokens as columns (gemm_columns.cu)."""
+    return bool(library().mx_gemm_columns_pays(m, n, k))
+
+
+def gemm_columns(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None,
+                 residual: torch.Tensor | None, out: torch.Tensor, mode: int,
+                 status: torch.Tensor | None = None) -> None:
+    """The product of some hundreds of rows on tcgen05 with the tokens as columns, in tiles that fill the rounds of the
+    SMs (operands as ``gemm_tcgen05`` takes them)."""
+    _need(a, "a", torch.bfloat16, contiguous=False)
+    _need(w, "w", torch.bfloat16)
+    _need(out, "out")
+    m, k = a.shape
+    n = w.shape[0]
+    assert w.shape[1] == k and tuple(out.shape) == (m, n), (a.shape, w.shape, out.shape)
+    if bias is not None:
+        _need(bias, "bias", torch.float32)
+        assert bias.numel() == n
+    if residual is not None:
+        _need(residual, "residual", torch.float32)
+        assert tuple(residual.shape) == (m, n) and residual.stride(0) == out.stride(0)
+    if status is None:
+        status = default_status(a.device)
+    check(library().mx_gemm_columns(_ptr(a), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out),
+                                    dtype_code(out.dtype), m, n, k, a.stride(0), w.stride(0),
+                                    out.stride(0), mode, _ptr(status), _stream()), "gemm_columns")
+    _launched()
+
+
 def gemm_tcgen05_force_tiles(rows: int) -> None:
     """Makes ``gemm_tcgen05`` use its 128-, 256- or 512-row kernel wherever the shape allows it; 0
     gives the choice back to the shape. For tests that run all three on the same product."""

@@ -44,6 +44,8 @@ _SIGNATURES: dict[str, tuple[list, object]] = {
     "mx_gemm_stream_pays": ([I, I, I], I),
     "mx_gemm_skinny_blocks": ([I, I, I], I),
     "mx_gemm_stream": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P, P], I),
+    "mx_gemm_columns_pays": ([I, I, I], I),
+    "mx_gemm_columns": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P, P], I),
     "mx_gemm_skinny": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P], I),
     "mx_gemm_skinny_rope": ([P, P, P, P, I, I, I, I, I, P, P, P, P, L, I, I, I, I, P, P], I),
     "mx_attention_scratch_bytes": ([I, I, I, I], L),

@@ -7,12 +7,13 @@ Backends, chosen by the runtime:
                matrix is streamed once and the epilogue is fused.
   "stream"  -- the engine's TMA + tcgen05 kernel for at most 128 rows with the tokens as the
                narrow side of the product: one block per SM streams its share of the weight rows.
-  "tcgen05" -- the engine's TMA + tcgen05 kernel for prompt-sized products: operands staged by
-               TMA, accumulator in tensor memory, epilogue fused.
+  "tcgen05" -- the engine's TMA + tcgen05 kernels for prompt-sized products with tiles of 128, 256 or 512
+               tokens: operands staged by TMA, accumulator in tensor memory, epilogue fused.
+  "columns" -- the same with the tokens as the columns of pairs of SMs, in tiles of any multiple of 16.
   "library" -- cuBLAS through ``torch.mm`` for bfloat16 (the reference runs its products
                through nn.Linear, i.e. the library: app/architectures/qwen_layers.py:50-53),
                followed by the engine's fused bias / GELU / residual epilogue kernel.
-  "auto"    -- for float32 "split" where it pays, else "simt"; for bfloat16 "skinny" up to 16 rows, "tcgen05" above 256 rows,
+  "auto"    -- for float32 "split" where it pays, else "simt"; for bfloat16 "skinny" up to 16 rows, "columns" or "tcgen05" above 256 rows,
                "library" between (a weight stream that 128-row tiles would leave to a few SMs) and
                for shapes neither takes (a K that is no multiple of 8), and "stream" from 9 rows
                on for large matrices (``_pick`` gives the measured thresholds).
@@ -55,7 +56,7 @@ def resolve_backend(requested: str, dtype: torch.dtype) -> str:
             raise KernelLibraryError(
                 f"the float32 path runs on the engine's float kernels only, not {requested!r}")
         return requested
-    if requested not in ("auto", "simt", "skinny", "stream", "tcgen05", "library"):
+    if requested not in ("auto", "simt", "skinny", "stream", "tcgen05", "columns", "library"):
         raise KernelLibraryError(f"unknown GEMM backend {requested!r}")
     return requested
 
@@ -86,7 +87,7 @@ def _pick(x: torch.Tensor, weight: torch.Tensor, m: int, n: int) -> str:
     # projections: 14 against 23 and 14 against 18 us at 512 rows), which have too few tiles to fill
     # the GPU and too little K to share out
     if m > 256 and kernels.tcgen05_gemm_supported(x, weight) and (m >= 1024 or n >= 8192 or x.shape[1] >= 8192):
-        return "tcgen05"
+        return "columns" if kernels.columns_gemm_pays(m, n, x.shape[1]) else "tcgen05"
     return "library"
 
 
@@ -174,6 +175,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, mod
         return out
     if backend == "stream":
         kernels.gemm_stream(x, weight, bias, residual, out, mode)
+        return out
+    if backend == "columns":
+        kernels.gemm_columns(x, weight, bias, residual, out, mode)
         return out
     if backend == "tcgen05":
         kernels.gemm_tcgen05(x, weight, bias, residual, out, mode)
