@@ -130,6 +130,7 @@ gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     if (warp == CL_EPI_WARPS) {
         // ---------------- producer (in both blocks): the whole warp walks, one elected lane issues
+        pdl_wait();
         int s = 0, it = 0;
         unsigned turn = 1;
         bool alive = true;
@@ -148,6 +149,7 @@ gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 if (++s == plan.stages) s = 0, turn ^= 1;
             }
         }
+        pdl_trigger();
         if (rank == 0)                                  // nothing stays in flight (the products read both blocks' stages)
             for (int j = max(0, it - plan.stages); j < it; ++j)
                 if (!tc_mbar_wait_warp(&sh.full[j % plan.stages], (unsigned)(j / plan.stages) & 1, status)) break;
@@ -182,6 +184,9 @@ gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     } else {
         // ---------------- epilogue: warp w has weight rows 32 (w % 4) .. of this block's 128 and half w / 4 of the tokens
         const int quarter = warp & 3, half = plan.tokens / 2, column = (warp >> 2) * half;
+        pdl_wait();                                     // the residual is somebody's output
+        residual = after_wait(residual);
+        bias = after_wait(bias);
         int local = 0;
         for (int item = pair; item < items; item += n_pairs, ++local) {
             int m0, n0, first, count;
@@ -336,9 +341,14 @@ extern "C" int mx_gemm_columns(const void* x, const void* W, const float* bias, 
     if (items > 0x3fffffffLL) MX_REFUSE("column gemm: %d x %d is beyond this kernel's grid", M, N);
     const int grid = 2 * (int)(items < pairs ? items : pairs);
     const size_t smem = 1024 + (size_t)plan.stages * (128 + plan.tokens / 2) * TC_BK * 2;
-    if (out_dtype == MX_DTYPE_F32)
-        gemm_columns_kernel<true><<<grid, CL_THREADS, smem, stream>>>(map_w, map_x, bias, residual, out, ldo, M, N, K, mode, plan, status);
-    else
-        gemm_columns_kernel<false><<<grid, CL_THREADS, smem, stream>>>(map_w, map_x, bias, residual, out, ldo, M, N, K, mode, plan, status);
-    return mx_launch_status();
+    const cudaError_t e = out_dtype == MX_DTYPE_F32
+                              ? mx_launch_chained(gemm_columns_kernel<true>, dim3(grid), dim3(CL_THREADS), smem, stream, map_w,
+                                                  map_x, bias, residual, out, ldo, M, N, K, mode, plan, status)
+                              : mx_launch_chained(gemm_columns_kernel<false>, dim3(grid), dim3(CL_THREADS), smem, stream, map_w,
+                                                  map_x, bias, residual, out, ldo, M, N, K, mode, plan, status);
+    if (e != cudaSuccess) {
+        mx_set_error("column gemm: launch failed: %s", cudaGetErrorString(e));
+        return (int)e;
+    }
+    return MX_OK;
 }
