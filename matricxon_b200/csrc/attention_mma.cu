@@ -74,6 +74,7 @@ struct MmaAttnParams {
     float cap_log2, cap_in;
     const float* sink;           // [heads] or null: exp(sink[h]) joins the softmax's denominator, with no value
     const float* distance;       // [2][heads] (r1, then r2) or null: scores lose r1 ln(1 + r2 (p - j))
+    int beside;                  // the next kernel starts beside this one and waits for nobody else (attention_tc.cu)
 };
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], unsigned a0, unsigned a1, unsigned a2,
@@ -246,7 +247,7 @@ attention_mma_kernel(const MmaAttnParams p) {
     __shared__ __align__(8) unsigned long long bars[N_STAGES];
     __shared__ int narrow_table[NARROW ? NARROW_TABLE : 1];   // the sequence's first block-table entries
 
-    pdl_trigger();
+    if (!p.beside) pdl_trigger();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int tile = blockIdx.x, kh = blockIdx.y, split = blockIdx.z;
@@ -347,6 +348,7 @@ attention_mma_kernel(const MmaAttnParams p) {
                              hi_tile, kept, bt, kbase, vbase, page_stride, lane, cached_for(0));
     // queries and the newest keys and values come from the kernels before this one
     pdl_wait();
+    if (p.beside) pdl_trigger();                        // what was waited for is now there for the next kernel too
     // Q fragments: 16 bytes of each owned row per 32-wide block. A row beyond the tile reads the
     // tile's last row (r_tok, r_head point there): its scores are masked and it is never written, and
     // a load that is not conditional is not waited for here.
@@ -765,7 +767,7 @@ extern "C" int mx_paged_attention_mma(const void* q, int q_stride, const void* c
                                       int n_heads, int n_kv_heads, int head_dim, int window,
                                       float scale, void* out, int out_stride, int n_splits,
                                       float* scratch, int* status, float softcap, const float* sink,
-                                      int keep_first, const float* distance, cudaStream_t stream) {
+                                      int keep_first, const float* distance, int beside, cudaStream_t stream) {
     if (n_tiles <= 0 || n_tokens <= 0) return MX_OK;
     if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0)
         MX_REFUSE("attention: %d heads are not a multiple of %d kv heads", n_heads, n_kv_heads);
@@ -794,6 +796,7 @@ extern "C" int mx_paged_attention_mma(const void* q, int q_stride, const void* c
     p.cap_in = softcap > 0.f ? scale / softcap : 0.f;
     p.sink = sink;
     p.distance = distance;
+    p.beside = beside;
     int rc;
     if (head_dim == 64) rc = narrow ? launch_mma<64, true>(p, stream) : launch_mma<64, false>(p, stream);
     else rc = narrow ? launch_mma<128, true>(p, stream) : launch_mma<128, false>(p, stream);

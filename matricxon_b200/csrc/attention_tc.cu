@@ -252,6 +252,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     // tiles start in the order of their list, which puts the ones with the most keys first, all heads of a tile side by
     // side (2,048 tokens, us in the list's order and from its end: 24 query heads on 2 KV heads 53 and 59, 16 on 16 32 and 41)
+    // (beside another kernel nothing is waited for here: what earlier kernels wrote is in memory, also for the copies below)
+    asm volatile("fence.proxy.async.global;\n" ::: "memory");
     const int tile = (int)(blockIdx.x / (unsigned)p.n_kv_heads);
     const int kh = (int)(blockIdx.x % (unsigned)p.n_kv_heads);
     const int seq = p.tiles[2 * tile], tok0 = p.tiles[2 * tile + 1];
@@ -672,6 +674,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
             }
         }
     }
+    // whoever waits for this kernel also waits for the one that it ran beside
+    pdl_wait();
     // ---------------- teardown: every role arrives here; then tensor memory is freed
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
@@ -727,7 +731,7 @@ extern "C" int mx_paged_attention_tc_split(const void* q, int q_stride, const vo
                                            int n_heads, int n_kv_heads, int head_dim, int window, float scale,
                                            void* out, int out_stride, int n_splits, float* scratch, int* status,
                                            float softcap, const float* sink, int keep_first, const float* distance,
-                                           cudaStream_t stream) {
+                                           int beside, cudaStream_t stream) {
     if (n_tiles <= 0 || n_tokens <= 0) return MX_OK;
     if (n_splits < 1 || n_splits > 64) MX_REFUSE("tcgen05 attention: %d key splits", n_splits);
     if (n_splits > 1 && scratch == nullptr) MX_REFUSE("tcgen05 attention: key splits without scratch memory");
@@ -741,6 +745,7 @@ extern "C" int mx_paged_attention_tc_split(const void* q, int q_stride, const vo
         reinterpret_cast<uintptr_t>(out) % 16 != 0 || reinterpret_cast<uintptr_t>(cache) % 16 != 0)
         MX_REFUSE("tcgen05 attention needs 16-byte aligned rows (strides %d, %d)", q_stride, out_stride);
     if (n_kv_heads > 65535) MX_REFUSE("attention: %d kv heads exceed the grid", n_kv_heads);
+    if (beside && n_splits > 1) MX_REFUSE("tcgen05 attention beside another kernel takes no key splits");
     if (status == nullptr) MX_REFUSE("tcgen05 attention needs a status word for its bounded waits");
     if (n_pages * 2 * n_kv_heads > 0x7fffffffLL) MX_REFUSE("tcgen05 attention: the cache has too many pages for a TMA coordinate");
     const int tokens_per_tile = AT_ROWS / group;
@@ -794,6 +799,19 @@ extern "C" int mx_paged_attention_tc_split(const void* q, int q_stride, const vo
     }
     if ((long long)n_tiles * n_kv_heads > 0x7fffffffLL) MX_REFUSE("tcgen05 attention: %d tiles exceed the grid", n_tiles);
     const dim3 grid((unsigned)(n_tiles * n_kv_heads), 1, n_splits);
+    if (beside) {
+        // The decoding requests' attention, launched just before, lets this kernel start once each of its blocks has seen
+        // the end of what both need (attention_mma.cu): the prompt's tiles then take the SMs that it leaves free, and those
+        // that its short requests give back. They wait for it only before they end. 31 requests of up to 6,000 tokens and a
+        // portion of 512 (7B sizes, 124 blocks there, 148 here): 2,513 us a step one after the other, 2,473 so.
+        const cudaError_t e = distance ? mx_launch_chained(attention_tc_kernel<true>, grid, dim3(AT_THREADS), smem, stream, q_map, k_map, v_map, p)
+                                       : mx_launch_chained(attention_tc_kernel<false>, grid, dim3(AT_THREADS), smem, stream, q_map, k_map, v_map, p);
+        if (e != cudaSuccess) {
+            mx_set_error("tcgen05 attention: launch failed: %s", cudaGetErrorString(e));
+            return (int)e;
+        }
+        return MX_OK;
+    }
     if (distance) attention_tc_kernel<true><<<grid, AT_THREADS, smem, stream>>>(q_map, k_map, v_map, p);
     else attention_tc_kernel<false><<<grid, AT_THREADS, smem, stream>>>(q_map, k_map, v_map, p);
     const int rc = mx_launch_status();
@@ -809,5 +827,5 @@ extern "C" int mx_paged_attention_tc(const void* q, int q_stride, const void* ca
                                      void* out, int out_stride, int* status, cudaStream_t stream) {
     return mx_paged_attention_tc_split(q, q_stride, cache, n_pages, page_size, block_tables, bt_stride, cu_q,
                                        context_lens, tiles, n_tiles, n_tokens, n_heads, n_kv_heads, head_dim, window,
-                                       scale, out, out_stride, 1, nullptr, status, 0.f, nullptr, 0, nullptr, stream);
+                                       scale, out, out_stride, 1, nullptr, status, 0.f, nullptr, 0, nullptr, 0, stream);
 }

@@ -539,13 +539,14 @@ def paged_attention_tc(q: torch.Tensor, q_stride: int, cache: torch.Tensor, bloc
                        scale: float, out: torch.Tensor, status: torch.Tensor, n_splits: int = 1,
                        scratch: torch.Tensor | None = None, softcap: float | None = None,
                        sink: torch.Tensor | None = None, keep_first: int = 0,
-                    distance: torch.Tensor | None = None) -> None:
+                    distance: torch.Tensor | None = None, beside: bool = False) -> None:
     """Attention of prompt portions on tcgen05 (bfloat16, head_dim 128, pages of 16 or 32). Under a window the
     sequence's first ``keep_first`` keys stay visible.
     ``tiles`` is int32 [n_tiles, 2]: (sequence, first token) of tiles of 128 // group tokens
     (``attention_tile_lists(..., token_tiles=True)``); ``q`` holds the step's rows, query head h
     at column h * head_dim. ``n_splits`` > 1 shares every tile's keys out between that many blocks
-    (few tiles, long contexts); ``scratch`` (float32, ``attention_scratch_bytes``) takes their parts."""
+    (few tiles, long contexts); ``scratch`` (float32, ``attention_scratch_bytes``) takes their parts. ``beside``: the
+    launch before this one is ``paged_attention_mma(..., beside=True)`` of the same step, and both run at a time."""
     _need(q, "q", torch.bfloat16, contiguous=False)
     _need(cache, "cache", torch.bfloat16)
     for name, tensor in (("block_tables", block_tables), ("cu_q", cu_q),
@@ -564,7 +565,7 @@ def paged_attention_tc(q: torch.Tensor, q_stride: int, cache: torch.Tensor, bloc
         block_tables.stride(0), _ptr(cu_q), _ptr(context_lens), _ptr(tiles), n_tiles, n_tokens,
         n_heads, n_kv_heads, head_dim, int(window or 0), float(scale), _ptr(out), out.stride(0),
         int(n_splits), _ptr(scratch) if n_splits > 1 else None, _ptr(status), float(softcap or 0.0),
-        _sink_ptr(sink, n_heads), int(keep_first) if window else 0, _distance_ptr(distance, n_heads), _stream()),
+        _sink_ptr(sink, n_heads), int(keep_first) if window else 0, _distance_ptr(distance, n_heads), int(beside), _stream()),
         "paged_attention_tc")
     _launched()
 
@@ -576,10 +577,10 @@ def paged_attention_mma(q: torch.Tensor, q_stride: int, cache: torch.Tensor,
                         out: torch.Tensor, status: torch.Tensor, n_splits: int = 1,
                         scratch: torch.Tensor | None = None, softcap: float | None = None,
                         sink: torch.Tensor | None = None, keep_first: int = 0,
-                    distance: torch.Tensor | None = None) -> None:
+                    distance: torch.Tensor | None = None, beside: bool = False) -> None:
     """Tensor-core attention (bfloat16, head_dim 64 or 128). ``tiles`` is int32 [n_tiles, 2]:
     (sequence, first row) of each tile of the (token, head-in-group) rows; ``narrow`` tiles
-    hold at most 16 rows, the others 64 (see ``attention_tile_lists``)."""
+    hold at most 16 rows, the others 64 (see ``attention_tile_lists``). ``beside``: ``paged_attention_tc(..., beside=True)`` follows."""
     _need(q, "q", torch.bfloat16, contiguous=False)
     _need(cache, "cache", torch.bfloat16)
     for name, tensor in (("block_tables", block_tables), ("cu_q", cu_q),
@@ -605,7 +606,7 @@ def paged_attention_mma(q: torch.Tensor, q_stride: int, cache: torch.Tensor,
         block_tables.stride(0), _ptr(cu_q), _ptr(context_lens), _ptr(tiles) if tiles is not None else None, n_tiles,
         1 if narrow else 0, n_tokens, n_heads, n_kv_heads, head_dim, int(window or 0), float(scale),
         _ptr(out), out.stride(0), n_splits, _ptr(scratch), _ptr(status), float(softcap or 0.0),
-        _sink_ptr(sink, n_heads), int(keep_first), _distance_ptr(distance, n_heads), _stream()), "paged_attention_mma")
+        _sink_ptr(sink, n_heads), int(keep_first), _distance_ptr(distance, n_heads), int(beside), _stream()), "paged_attention_mma")
     _launched(2 if n_splits > 1 else 1)
 
 

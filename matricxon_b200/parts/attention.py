@@ -149,6 +149,8 @@ def paged_attend(q, q_stride, ctx, binding, rt, n_heads, n_kv_heads, head_dim, w
         # prompt portions on tcgen05 when the kernel takes the geometry, else on mma.sync
         on_tc = _TC_ATTENTION and kernels.tc_attention_supported(rt.dtype, head_dim, rt.page_size, q_stride, group_size)
         narrow, n_narrow, wide, n_wide = attention_tiles(ctx, group_size, token_tiles=on_tc)
+        # decoding requests and prompt portions in one step: their two kernels run at a time
+        beside = on_tc and n_narrow > 0 and n_wide > 0
         for tiles, n_tiles, is_narrow in ((narrow, n_narrow, True), (wide, n_wide, False)):
             if n_tiles == 0:
                 continue
@@ -159,7 +161,7 @@ def paged_attend(q, q_stride, ctx, binding, rt, n_heads, n_kv_heads, head_dim, w
                                            ctx.context_lens, tiles, n_tiles, ctx.n_tokens,
                                            n_heads, n_kv_heads, head_dim,
                                            window, scale, attn, ctx.status,
-                                           n_splits=n_splits, scratch=scratch, **extras, **kept)
+                                           n_splits=n_splits, scratch=scratch, beside=beside, **extras, **kept)
                 continue
             alone = (n_wide == 0) if is_narrow else (n_narrow == 0)
             if is_narrow and ctx.padded:
@@ -170,7 +172,7 @@ def paged_attend(q, q_stride, ctx, binding, rt, n_heads, n_kv_heads, head_dim, w
                                         ctx.cu_q, ctx.context_lens, tiles, n_tiles, is_narrow,
                                         ctx.n_tokens, n_heads, n_kv_heads,
                                         head_dim, window, scale, attn, ctx.status,
-                                        n_splits=n_splits, scratch=scratch, **extras, **kept)
+                                        n_splits=n_splits, scratch=scratch, beside=beside, **extras, **kept)
     else:
         n_splits, scratch = simt_splits(ctx, n_heads, n_kv_heads,
                                                  head_dim, span)
