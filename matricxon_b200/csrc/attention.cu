@@ -315,7 +315,8 @@ paged_attention_kernel(const AttnParams p) {
 // by side (four numbers a lane; scores are summed over the lanes by halving, sixteen keys at once), and a lane takes four
 // value dimensions of sixteen slots, 64 bytes each. The four warps of a block walk the chunks of its share in turn, each
 // with a softmax of its own, and are combined at the end. Bound by the multiply-adds of long prompts (two thirds of the
-// instructions) and by one trip to memory in decoding.
+// instructions) and by one trip to memory in decoding. Steps of eight layers at the 3B sizes: a prompt of 389 tokens 5,806 ->
+// 5,131 us, four requests of 490 to 701 tokens 1,581 -> 1,397.
 constexpr int F32A_KEYS = 16, F32A_DIM = 128;
 
 __device__ __forceinline__ void load8(const float* p, float* v) {

@@ -6,7 +6,8 @@
 // h h, h m, m h, m m, h l, l h; what is left out is below 2^-26 of a term. The tensor cores add in float but cut sums off
 // instead of rounding them, so an accumulator only ever holds 32 values of k, the small products first and h h last; it is
 // then added to float registers, rounded to nearest (96 additions for K = 3,072, where the FP32 cores' chains make 768 to a
-// piece).
+// piece). Root mean square error against 64 bits, of the result's: 1.1e-7 to 1.9e-7 for K = 3,072 (by the shares of K; the FP32
+// cores 5.0e-7), 1.8e-7 to 3.6e-7 for K = 12,288 (1.0e-6).
 // A result that is not finite (an operand that is not, an overflow on the way, a float above bfloat16's largest) is formed
 // again from the operands by plain multiply-adds, which decide what it is. The reference runs these products through
 // nn.Linear (app/architectures/qwen_layers.py:50-53, app/architectures/starcoder2_layers.py:19-23).
@@ -17,7 +18,11 @@
 // a cycle then bound products of few tokens, a stage took 1,000 cycles). Up to 64 tokens of a tile are split
 // beside them; more are split once, by a kernel of their own, and come by TMA as parts. Eight more warps add up the
 // accumulators, of which there are two to four. K is dealt out to the blocks of a cluster where tiles alone leave SMs idle;
-// each block finishes a share of the tokens from all sums, in the order of K.
+// each block finishes a share of the tokens from all sums, in the order of K. 389 rows x 12,288 x 3,072 and 3,072 x 12,288 take
+// 170 and 166 us (the FP32 cores 701 and 790), 1,024 rows 362 and 352 (1,589 and 1,625), 64 rows 69 and 61 (136 and 298): 172 to
+// 220 TFLOP/s of the 278 that six products leave of the measured rate. What is left is a tile's start and end, about 13,000
+// cycles beside 96 stages of 1,300. With splitting and adding in the same eight warps a stage took 1,600 to 1,850 cycles
+// whatever its size, with one issuer 5 % more than with two.
 #include <cooperative_groups.h>
 
 #include "common.cuh"

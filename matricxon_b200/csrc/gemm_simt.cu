@@ -1,13 +1,14 @@
 // out[M,N] = epilogue(A[M,K] . W[N,K]^T + bias[N]) on the FP32 cores.
 //
-// This is the true 32-bit matrix product of the engine (inputs, products and sums are
-// float; no tensor-core mode), and the plain twin that the tensor-core product is checked
-// against. Each output element is one fixed-order sum over K, whatever M is, so a row's
-// result does not depend on what else is in the batch: four chains over a quarter of K each, added
-// as (p0 + p1) + (p2 + p3) (gemm_f32.cuh; one chain over all of K leaves few threads to a decoding
-// row, and its rounding errors are twice as large). Float operands that can be read 16 bytes at a
-// time go to gemm_f32.cu, which forms the same sums. The reference runs these products
-// through nn.Linear (app/architectures/qwen_layers.py:50-53,
+// This is the plain 32-bit matrix product of the engine (inputs, products and sums are
+// float), and the twin that the tensor-core products are checked against, those of floats
+// in three parts (gemm_f32_split.cu, which takes the larger products of three rows and
+// more) among them. Each output element is one fixed-order sum over K, whatever M is, so a
+// row's result does not depend on what else is in the batch: four chains over a quarter of K
+// each, added as (p0 + p1) + (p2 + p3) (gemm_f32.cuh; one chain over all of K leaves few
+// threads to a decoding row, and its rounding errors are twice as large). Float operands
+// that can be read 16 bytes at a time go to gemm_f32.cu, which forms the same sums. The
+// reference runs these products through nn.Linear (app/architectures/qwen_layers.py:50-53,
 // app/architectures/starcoder2_layers.py:19-23).
 //
 // Epilogue modes: 0 out(T) = v; 1 out(T) = gelu_tanh(v); 2 out(f32) = residual + v;
