@@ -314,9 +314,12 @@ paged_attention_kernel(const AttnParams p) {
 // page) for the token's heads of one KV head, and what it loads goes straight to registers: a key's row is 512 bytes side
 // by side (four numbers a lane; scores are summed over the lanes by halving, sixteen keys at once), and a lane takes four
 // value dimensions of sixteen slots, 64 bytes each. The four warps of a block walk the chunks of its share in turn, each
-// with a softmax of its own, and are combined at the end. Bound by the multiply-adds of long prompts (two thirds of the
+// with a softmax of its own, and are combined at the end. Up to six heads a block, so that four blocks fit an SM: eight warps
+// of twelve heads hide too little (a prompt of 389 tokens, 24 heads on 2: 126 us, 100 with six; 200 tokens, 16 on 2: 39 and
+// 30), though keys and values are then read twice. Bound by the multiply-adds of long prompts (two thirds of the
 // instructions) and by one trip to memory in decoding. Steps of eight layers at the 3B sizes: a prompt of 389 tokens 5,806 ->
-// 5,131 us, four requests of 490 to 701 tokens 1,581 -> 1,397.
+// 5,131 us, four requests of 490 to 701 tokens 1,581 -> 1,397; with six heads a block and the split products for few rows 5,221
+// -> 5,111 and 1,108 -> 1,071.
 constexpr int F32A_KEYS = 16, F32A_DIM = 128;
 
 __device__ __forceinline__ void load8(const float* p, float* v) {
@@ -327,11 +330,12 @@ __device__ __forceinline__ void load8(const float* p, float* v) {
 
 // HEADS: query heads of a block, padded.
 template <int HEADS>
-__global__ void __launch_bounds__(ATT_THREADS)
+__global__ void __launch_bounds__(ATT_THREADS, 4)
 paged_attention_f32_kernel(const AttnParams p) {
     __shared__ float4 weights[ATT_WARPS][HEADS][F32A_KEYS / 4];
     __shared__ float sums[ATT_WARPS][HEADS][F32A_DIM];
     __shared__ float maxima[ATT_WARPS][HEADS], totals[ATT_WARPS][HEADS];
+    __shared__ float4 queries[HEADS][F32A_DIM / 4];     // in registers they would cost an SM one of its four blocks
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.x, split = blockIdx.z;
     const int group = p.n_heads / p.n_kv_heads, n_hgroups = (group + HEADS - 1) / HEADS;
@@ -366,17 +370,18 @@ paged_attention_f32_kernel(const AttnParams p) {
     const int* bt = p.block_tables + (size_t)seq * p.bt_stride;
     const size_t head_stride = (size_t)p.page_size * F32A_DIM;
 
-    float4 qv[HEADS];
     float acc[HEADS][4], m_run[HEADS], l_run[HEADS];                       // l_run: of this lane's keys
 #pragma unroll
     for (int h = 0; h < HEADS; ++h) {
-        qv[h] = h < heads ? reinterpret_cast<const float4*>(q + (size_t)t * p.q_stride + (size_t)(head0 + h) * F32A_DIM)[lane]
-                          : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (h % ATT_WARPS == warp)
+            queries[h][lane] = h < heads ? reinterpret_cast<const float4*>(q + (size_t)t * p.q_stride + (size_t)(head0 + h) * F32A_DIM)[lane]
+                                         : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[h][i] = 0.f;
         m_run[h] = -INFINITY;
         l_run[h] = 0.f;
     }
+    __syncthreads();
     for (int c = c_begin + warp; c < c_end; c += ATT_WARPS) {
         const int c0 = (c < n_kept ? c : first_chunk + c - n_kept) * F32A_KEYS;
         const int lp = c0 / p.page_size, off = c0 - lp * p.page_size;
@@ -401,9 +406,10 @@ paged_attention_f32_kernel(const AttnParams p) {
 #pragma unroll
         for (int h = 0; h < HEADS; ++h) {
             float s[F32A_KEYS];
+            const float4 qv = queries[h][lane];
 #pragma unroll
             for (int j = 0; j < F32A_KEYS; ++j)
-                s[j] = fmaf(qv[h].w, kv[j].w, fmaf(qv[h].z, kv[j].z, fmaf(qv[h].y, kv[j].y, qv[h].x * kv[j].x)));
+                s[j] = fmaf(qv.w, kv[j].w, fmaf(qv.z, kv[j].z, fmaf(qv.y, kv[j].y, qv.x * kv[j].x)));
 #pragma unroll
             for (int half = F32A_KEYS / 2; half > 0; half >>= 1) {
                 const bool upper = lane & (2 * half);
@@ -682,10 +688,8 @@ int launch_attention(const AttnParams& p, int n_tokens, cudaStream_t stream) {
     dim3 grid(n_tokens, p.n_kv_heads * n_hgroups, p.n_splits);
     int rc;
     if (sixteen_keys_a_warp<T>(p)) {
-        const int parts = (group + 11) / 12, heads = (group + parts - 1) / parts;       // of a block, evenly dealt
-        rc = heads <= 4 ? launch_attention_f32<4>(p, n_tokens, stream)
-             : heads <= 8 ? launch_attention_f32<8>(p, n_tokens, stream)
-                          : launch_attention_f32<12>(p, n_tokens, stream);
+        const int parts = (group + 5) / 6, heads = (group + parts - 1) / parts;         // of a block, evenly dealt
+        rc = heads <= 4 ? launch_attention_f32<4>(p, n_tokens, stream) : launch_attention_f32<6>(p, n_tokens, stream);
     } else {
         paged_attention_kernel<T, HD_SLOTS><<<grid, ATT_THREADS, smem, stream>>>(p);
         rc = mx_launch_status();
