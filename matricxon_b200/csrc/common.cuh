@@ -42,6 +42,11 @@ static inline int mx_launch_status() {
     return MX_OK;
 }
 
+// Parts of K that a product's sums may be left in, added up by whoever reads them (gemm_columns.cu, elementwise.cu).
+#define MX_SUM_PARTS 8
+extern "C" int mx_add_parts(const float* parts, int ldp, int n_parts, const float* bias, float* out, int ldo, int M, int N,
+                            cudaStream_t stream);
+
 // ---- programmatic dependent launch: a kernel launched with mx_launch_chained may start while the
 // kernel before it in the stream is still running. It must call pdl_wait() before it reads anything
 // an earlier kernel wrote and before it writes global memory at all; what it does before that

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(LN_THREADS)
 layernorm_vec_kernel(const float* x, const int* __restrict__ rows,
                      const float* __restrict__ weight, const float* __restrict__ bias,
                      TOut* __restrict__ out, int hidden, float eps, const float* acc, const float* col_bias,
-                     float* x_sum) {
+                     float* x_sum, int n_parts, size_t plane) {
     __shared__ float scratch[32];
     pdl_trigger();
     const int r = blockIdx.x;
@@ -187,20 +187,32 @@ layernorm_vec_kernel(const float* x, const int* __restrict__ rows,
         const float4* ar = reinterpret_cast<const float4*>(after_wait(acc) + (size_t)src_row * hidden);
         const float4* cb = reinterpret_cast<const float4*>(col_bias);
         float4* xw = reinterpret_cast<float4*>(after_wait(x_sum) + (size_t)src_row * hidden);
+        // a tensor at a time, a thread's vectors of it together: the loads of one are out before the first is added
+        auto add_row = [&](const float4* from) {
+            float4 more[LN_VPT];
+#pragma unroll
+            for (int k = 0; k < LN_VPT; ++k) {
+                const int i = threadIdx.x + k * LN_THREADS;
+                more[k] = i < n_vec ? from[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < LN_VPT; ++k) {
+                v[k].x += more[k].x; v[k].y += more[k].y; v[k].z += more[k].z; v[k].w += more[k].w;
+            }
+        };
 #pragma unroll
         for (int k = 0; k < LN_VPT; ++k) {
             const int i = threadIdx.x + k * LN_THREADS;
-            v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i < n_vec) {
-                float4 a = ar[i];
-                const float4 r = xr[i];
-                if (col_bias) {
-                    const float4 b = cb[i];
-                    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-                }
-                v[k] = make_float4(a.x + r.x, a.y + r.y, a.z + r.z, a.w + r.w);
-                xw[i] = v[k];
-            }
+            v[k] = i < n_vec ? ar[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        for (int p = 1; p < n_parts; ++p)               // the product's parts of K, in their order
+            add_row(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(ar) + p * plane));
+        if (col_bias) add_row(cb);
+        add_row(xr);
+#pragma unroll
+        for (int k = 0; k < LN_VPT; ++k) {
+            const int i = threadIdx.x + k * LN_THREADS;
+            if (i < n_vec) xw[i] = v[k];
             s += (v[k].x + v[k].y) + (v[k].z + v[k].w);
         }
     } else {
@@ -251,12 +263,13 @@ extern "C" int mx_epilogue(const void* acc, int acc_dtype, const float* bias, co
                            int out_dtype, long long n_rows, int n_cols, int mode, cudaStream_t stream);
 
 // acc != null: x (float, written) first becomes x + acc + col_bias (the residual epilogue of the product
-// whose float accumulator acc is), in the same launch where the rows allow 16-byte accesses, else by the
+// whose float accumulator acc is, or the n_parts parts of it, [n_parts][n_rows][hidden]), in the same launch where the rows allow 16-byte accesses, else by the
 // epilogue kernel ahead of the norm. rows must be null then.
 static int layernorm_launch(float* x_sum, const float* x, const int* rows, const float* weight, const float* bias,
                             void* out, int out_dtype, int n_rows, int hidden, float eps, const float* acc,
-                            const float* col_bias, cudaStream_t stream) {
+                            const float* col_bias, cudaStream_t stream, int n_parts = 1) {
     if (n_rows <= 0) return MX_OK;
+    const size_t plane = (size_t)n_rows * hidden;
     const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(weight) |
                            reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(out) |
                            reinterpret_cast<uintptr_t>(acc) | reinterpret_cast<uintptr_t>(col_bias)) & 15) == 0;
@@ -273,7 +286,7 @@ static int layernorm_launch(float* x_sum, const float* x, const int* rows, const
         if (n_rows <= 256) threads = n_vec <= 256 ? 256 : (n_vec <= 512 ? 512 : (n_vec <= 768 ? 768 : 1024));
 #define MX_LN_LAUNCH(T, N)                                                                                       \
     mx_launch_chained(layernorm_vec_kernel<T, N>, dim3(n_rows), dim3(N), 0, stream, x, rows, weight, bias, (T*)out, \
-                      hidden, eps, acc, col_bias, x_sum)
+                      hidden, eps, acc, col_bias, x_sum, n_parts, plane)
         if (out_dtype == MX_DTYPE_F32) {
             if (threads == 64) MX_LN_LAUNCH(float, 64);
             else if (threads == 96) MX_LN_LAUNCH(float, 96);
@@ -297,7 +310,8 @@ static int layernorm_launch(float* x_sum, const float* x, const int* rows, const
         return mx_launch_status();
     }
     if (acc != nullptr) {       // the general kernel takes a finished row: the sum is formed by the epilogue kernel
-        const int rc = mx_epilogue(acc, MX_DTYPE_F32, col_bias, x, x_sum, MX_DTYPE_F32, n_rows, hidden, 2, stream);
+        const int rc = n_parts > 1 ? mx_add_parts(acc, hidden, n_parts, col_bias, x_sum, hidden, n_rows, hidden, stream)
+                                   : mx_epilogue(acc, MX_DTYPE_F32, col_bias, x, x_sum, MX_DTYPE_F32, n_rows, hidden, 2, stream);
         if (rc != MX_OK) return rc;
     }
     const size_t smem = (size_t)hidden * sizeof(float);
@@ -325,12 +339,64 @@ extern "C" int mx_layernorm(const float* x, const int* rows, const float* weight
 }
 
 // x <- x + acc + col_bias (col_bias may be null), then out <- LayerNorm(x): the residual epilogue of a
-// product and the norm after it in one pass over the rows.
-extern "C" int mx_layernorm_sum(float* x, const float* acc, const float* col_bias, const float* weight,
+// product and the norm after it in one pass over the rows. acc may be left in parts of K, [n_parts][n_rows][hidden].
+extern "C" int mx_layernorm_sum(float* x, const float* acc, int n_parts, const float* col_bias, const float* weight,
                                 const float* bias, void* out, int out_dtype, int n_rows, int hidden, float eps,
                                 cudaStream_t stream) {
     if (acc == nullptr) MX_REFUSE("layernorm with sum: no accumulator");
-    return layernorm_launch(x, x, nullptr, weight, bias, out, out_dtype, n_rows, hidden, eps, acc, col_bias, stream);
+    if (n_parts < 1 || n_parts > MX_SUM_PARTS) MX_REFUSE("layernorm with sum: %d parts", n_parts);
+    return layernorm_launch(x, x, nullptr, weight, bias, out, out_dtype, n_rows, hidden, eps, acc, col_bias, stream,
+                            n_parts);
+}
+
+// out[m][n] += bias[n] + the sums of a product's parts of K, added in their order (gemm_columns.cu).
+constexpr int PARTS_THREADS = 256;
+template <int WIDTH>
+__global__ void __launch_bounds__(PARTS_THREADS)
+add_parts_kernel(const float* __restrict__ parts, int ldp, int splits, const float* __restrict__ bias, float* out, int ldo,
+                     int M, int N) {
+    pdl_trigger();
+    const int per_row = (N + WIDTH - 1) / WIDTH;
+    const long long i = (long long)blockIdx.x * PARTS_THREADS + threadIdx.x;
+    pdl_wait();
+    parts = after_wait(parts);
+    bias = after_wait(bias);
+    if (i >= (long long)per_row * M) return;
+    const int m = (int)(i / per_row), n = (int)(i - (long long)m * per_row) * WIDTH;
+    const size_t plane = (size_t)M * ldp;
+    const float* from = parts + (size_t)m * ldp + n;
+    float* to = out + (size_t)m * ldo + n;
+    if constexpr (WIDTH == 4) {
+        float4 part[MX_SUM_PARTS];
+#pragma unroll
+        for (int s = 0; s < MX_SUM_PARTS; ++s)
+            if (s < splits) part[s] = __ldcg(reinterpret_cast<const float4*>(from + s * plane));
+        const float4 old = *reinterpret_cast<const float4*>(to);
+        const float4 b = bias != nullptr ? make_float4(bias[n], bias[n + 1], bias[n + 2], bias[n + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 v = part[0];
+#pragma unroll
+        for (int s = 1; s < MX_SUM_PARTS; ++s)
+            if (s < splits) v.x += part[s].x, v.y += part[s].y, v.z += part[s].z, v.w += part[s].w;
+        *reinterpret_cast<float4*>(to) = make_float4(v.x + b.x + old.x, v.y + b.y + old.y, v.z + b.z + old.z, v.w + b.w + old.w);
+    } else {
+        float v = __ldcg(from);
+        for (int s = 1; s < splits; ++s) v += __ldcg(from + s * plane);
+        *to = v + (bias != nullptr ? bias[n] : 0.f) + *to;
+    }
+}
+
+extern "C" int mx_add_parts(const float* parts, int ldp, int n_parts, const float* bias, float* out, int ldo, int M, int N,
+                            cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return MX_OK;
+    if (n_parts < 1 || n_parts > MX_SUM_PARTS) MX_REFUSE("add parts: %d parts", n_parts);
+    const bool wide = N % 4 == 0 && ldo % 4 == 0 && ldp % 4 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(parts)) & 15) == 0;
+    const long long blocks = ((long long)M * (wide ? N / 4 : N) + PARTS_THREADS - 1) / PARTS_THREADS;
+    if (blocks > 0x7fffffffLL) MX_REFUSE("add parts: %d x %d is beyond the grid", M, N);
+    if (wide)
+        mx_launch_chained(add_parts_kernel<4>, dim3((unsigned)blocks), dim3(PARTS_THREADS), 0, stream, parts, ldp, n_parts, bias, out, ldo, M, N);
+    else
+        mx_launch_chained(add_parts_kernel<1>, dim3((unsigned)blocks), dim3(PARTS_THREADS), 0, stream, parts, ldp, n_parts, bias, out, ldo, M, N);
+    return mx_launch_status();
 }
 
 // ---------------------------------------------------------------- rotary + cache write

@@ -7,8 +7,13 @@
 // tiles of 192. A pair of blocks owns 256 weight rows of a tile (cta_group::2: each block its 128 rows and half of the
 // tokens, so 16 KB + 64 bytes a token for 64 of K), a ring of TMA stages feeds it through its tiles without a break, and two
 // accumulators let the eight epilogue warps of a block store one tile under the next one's products. Where the result is a
-// sum added to the stream in place, K is also shared out: the parts add to memory (in no fixed order, as in the kernel for
-// 256-row tiles). The reference runs these products through nn.Linear (app/architectures/qwen_layers.py:50-53,
+// sum added to the stream in place, K is also shared out: every part leaves its sums in scratch memory, and whoever reads the
+// stream next (the norm, mx_layernorm_sum), or else a kernel of its own, adds them in the order of K, so that a product
+// repeats bit by bit. Product and norm, us, against adding to memory in the order in which the parts end, which does not
+// repeat: 367 x 3,072 x 12,288 35.2 and 33.1, 512 rows 40.6 and 39.3, 1,024 x 1,024 x 6,144 21.2 and 21.2, 2,048 rows 30.0 and
+// 30.7 (35 to 44 with K in one piece); parts that meet in the shared memory of clusters of four or six blocks take 3 to 7 us
+// more, since 66 pairs run at a time then instead of 74.
+// The reference runs these products through nn.Linear (app/architectures/qwen_layers.py:50-53,
 // app/architectures/starcoder2_layers.py:19-23).
 #include <stdlib.h>
 
@@ -20,6 +25,7 @@ namespace {
 constexpr int CL_ROWS = 256, CL_TOKENS = 256;           // weight rows of a pair's tile; tokens of it at most
 constexpr int CL_EPI_WARPS = 8, CL_THREADS = 32 * (CL_EPI_WARPS + 2);
 constexpr int CL_MAX_STAGES = 8, CL_SMEM = 220 * 1024;
+constexpr int CL_MAX_SPLITS = MX_SUM_PARTS;             // parts of K
 
 struct ClPlan {
     int tokens, token_tiles;    // a multiple of 16; how many such tiles
@@ -85,7 +91,7 @@ template <bool F32>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CL_THREADS, 1)
 gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     const float* __restrict__ bias, const float* residual, void* out, int ldo, int M, int N, int K, int mode,
-                    const ClPlan plan, int* status) {
+                    const ClPlan plan, float* parts, int ldp, int* status) {
     extern __shared__ unsigned char cl_smem_raw[];
     unsigned char* ring = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(cl_smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -192,11 +198,11 @@ gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             int m0, n0, first, count;
             place(item, m0, n0, first, count);
             const int b = local & 1, n = n0 + 128 * (int)rank + 32 * quarter + lane;
-            const bool mine = n < N, adds = F32 && plan.splits > 1;
-            const float bias_here = mine && bias != nullptr && first == 0 ? bias[n] : 0.f;
+            const bool mine = n < N, shared = F32 && plan.splits > 1;       // a part of K: its sums alone, to scratch memory
+            const float bias_here = mine && bias != nullptr && !shared ? bias[n] : 0.f;
             const int tokens = min(half, M - m0 - column);                  // of this warp
             // sixteen tokens at a time; what a sum in place is added to sets out sixteen tokens ahead
-            const float* old = F32 && mode == MX_MODE_RESIDUAL && !adds && mine ? residual + (size_t)(m0 + column) * ldo + n : nullptr;
+            const float* old = F32 && mode == MX_MODE_RESIDUAL && !shared && mine ? residual + (size_t)(m0 + column) * ldo + n : nullptr;
             float before[16];
             auto fetch = [&](int c) {
 #pragma unroll
@@ -206,12 +212,14 @@ gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             if (!tc_mbar_wait_warp(&sh.acc_full[b], (unsigned)(local >> 1) & 1, status)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const unsigned from = tmem_base + (unsigned)(b * CL_TOKENS + column) + ((unsigned)(32 * quarter) << 16);
+            float* const to_f32 = shared ? parts + (size_t)(first / per) * M * ldp : reinterpret_cast<float*>(out);
+            const int stride = shared ? ldp : ldo;
             for (int c = 0; c < tokens; c += 16) {
                 unsigned r[16];
                 tmem_load16(from + (unsigned)c, r);
-                const size_t o = (size_t)(m0 + column + c) * ldo + n;
+                const size_t o = (size_t)(m0 + column + c) * stride + n;
                 if constexpr (F32) {
-                    float* to = reinterpret_cast<float*>(out) + o;
+                    float* to = to_f32 + o;
                     float sum[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j) sum[j] = __uint_as_float(r[j]) + bias_here + before[j];
@@ -220,8 +228,7 @@ gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         if (c + j >= tokens) break;
-                        if (adds) asm volatile("red.global.add.f32 [%0], %1;\n" ::"l"(to + (size_t)j * ldo), "f"(sum[j]) : "memory");
-                        else to[(size_t)j * ldo] = sum[j];
+                        to[(size_t)j * stride] = sum[j];
                     }
                 } else {
                     if (!mine) continue;
@@ -271,7 +278,8 @@ int cl_pairs() {
 
 // Tiles, parts of K and the cycles that they take: a slice of 64 of K takes a pair the longer of its products (2 cycles a
 // token) and its loads (53 bytes a cycle and SM); an item costs the turn from one accumulator to the next, the launch its
-// start and the last item's stores, and sums added in memory take what L2 adds in a cycle (1,100 bytes).
+// start and the last item's stores; the sums of a part are 4 bytes a result to write and to read again, and less of an item's
+// end is hidden (480 x 6,144 x 24,576 in three parts 117 us, in one 110; 2,048 x 1,024 x 6,144 in two 30, in one 35).
 double cl_plan(int M, int N, int K, bool may_split, int pairs, ClPlan* best) {
     double best_cost = -1.0;
     const int weight_tiles = (N + CL_ROWS - 1) / CL_ROWS, slices = (K + TC_BK - 1) / TC_BK;
@@ -280,12 +288,12 @@ double cl_plan(int M, int N, int K, bool may_split, int pairs, ClPlan* best) {
         const int tokens = ((M + tiles - 1) / tiles + 15) / 16 * 16;
         if (tiles > least && tokens * (tiles - 1) >= M) continue;
         const double slice = max(2.0 * tokens, (16384.0 + 64.0 * tokens) / 53.0);
-        for (int splits = 1; splits <= (may_split ? 8 : 1); ++splits) {
+        for (int splits = 1; splits <= (may_split ? CL_MAX_SPLITS : 1); ++splits) {
             const int per = (slices + splits - 1) / splits;
             if (splits > 1 && (per < 8 || (splits - 1) * per >= slices)) continue;
             const long long rounds = ((long long)weight_tiles * tiles * splits + pairs - 1) / pairs;
-            double cost = rounds * (per * slice + 500.0) + 4000.0 + 20.0 * tokens;
-            if (splits > 1) cost += 4.0 * M * N * splits / 1100.0;
+            double cost = rounds * (per * slice + (splits > 1 ? 2500.0 : 500.0)) + 4000.0 + 20.0 * tokens;
+            if (splits > 1) cost += 4.0 * M * N * (splits + 1.0) / 1400.0;
             if (best_cost < 0.0 || cost < best_cost) {
                 best_cost = cost;
                 best->tokens = tokens;
@@ -311,8 +319,33 @@ extern "C" int mx_gemm_columns_pays(int M, int N, int K) {
     return M > 256 && !(M >= 2048 && N < K && K >= (M >= 8192 ? 6144 : M >= 4096 ? 8192 : 12288));
 }
 
+namespace {
+
+// The plan of a product; `in_place`: its result is a sum added to the stream in place. MATRICXON_GEMM_SPLIT_K=0 keeps every
+// tile's K in one pair.
+ClPlan cl_plan_of(int M, int N, int K, bool in_place, int pairs) {
+    static const bool split_allowed = [] {
+        const char* env = getenv("MATRICXON_GEMM_SPLIT_K");
+        return env == nullptr || env[0] != '0';
+    }();
+    ClPlan plan = {};
+    cl_plan(M, N, K, in_place && split_allowed, pairs, &plan);
+    return plan;
+}
+
+}  // namespace
+
+// Parts of K that a product added to the stream in place is cut into (1: none), each [M][N rounded up to 4] floats of scratch.
+extern "C" int mx_gemm_columns_parts(int M, int N, int K) {
+    const int pairs = M > 0 && N > 0 && K > 0 ? cl_pairs() : 0;
+    return pairs > 0 ? cl_plan_of(M, N, K, true, pairs).splits : 1;
+}
+
+// `parts`: the scratch memory of a product that is added to the stream in place and cut into parts of K; null otherwise. With
+// `finish` 0 the sums stay there (out and bias are not touched) for mx_layernorm_sum or mx_add_parts.
 extern "C" int mx_gemm_columns(const void* x, const void* W, const float* bias, const float* residual, void* out, int out_dtype,
-                               int M, int N, int K, int ldx, int ldw, int ldo, int mode, int* status, cudaStream_t stream) {
+                               float* parts, int finish, int M, int N, int K, int ldx, int ldw, int ldo, int mode, int* status,
+                               cudaStream_t stream) {
     if (M <= 0 || N <= 0) return MX_OK;
     if (K <= 0 || K % 8 != 0) MX_REFUSE("column gemm: K = %d is not a positive multiple of 8", K);
     if (ldx % 8 != 0 || ldw % 8 != 0) MX_REFUSE("column gemm: row strides %d, %d are not multiples of 8", ldx, ldw);
@@ -325,13 +358,9 @@ extern "C" int mx_gemm_columns(const void* x, const void* W, const float* bias, 
     if (status == nullptr) MX_REFUSE("column gemm: a status word is needed for its bounded waits");
     const int pairs = cl_pairs();
     if (pairs <= 0) MX_REFUSE("column gemm: pairs of SMs cannot run %d bytes of shared memory", CL_SMEM);
-    // MATRICXON_GEMM_SPLIT_K=0 keeps every tile's K in one pair: sums added in memory may differ in the last bit from run to run
-    static const bool split_allowed = [] {
-        const char* env = getenv("MATRICXON_GEMM_SPLIT_K");
-        return env == nullptr || env[0] != '0';
-    }();
-    ClPlan plan = {};
-    cl_plan(M, N, K, mode == MX_MODE_RESIDUAL && residual == out && split_allowed, pairs, &plan);
+    const ClPlan plan = cl_plan_of(M, N, K, mode == MX_MODE_RESIDUAL && residual == out, pairs);
+    if (plan.splits > 1 && (parts == nullptr || (reinterpret_cast<uintptr_t>(parts) & 15)))
+        MX_REFUSE("column gemm: %d parts of K need scratch on a 16-byte boundary", plan.splits);
     CUtensorMap map_w, map_x;
     int rc = mx_tensor_map_2d(&map_w, W, N, K, ldw, 128);
     if (rc != MX_OK) return rc;
@@ -341,14 +370,17 @@ extern "C" int mx_gemm_columns(const void* x, const void* W, const float* bias, 
     if (items > 0x3fffffffLL) MX_REFUSE("column gemm: %d x %d is beyond this kernel's grid", M, N);
     const int grid = 2 * (int)(items < pairs ? items : pairs);
     const size_t smem = 1024 + (size_t)plan.stages * (128 + plan.tokens / 2) * TC_BK * 2;
+    const int ldp = (N + 3) / 4 * 4;
     const cudaError_t e = out_dtype == MX_DTYPE_F32
                               ? mx_launch_chained(gemm_columns_kernel<true>, dim3(grid), dim3(CL_THREADS), smem, stream, map_w,
-                                                  map_x, bias, residual, out, ldo, M, N, K, mode, plan, status)
+                                                  map_x, bias, residual, out, ldo, M, N, K, mode, plan, parts, ldp, status)
                               : mx_launch_chained(gemm_columns_kernel<false>, dim3(grid), dim3(CL_THREADS), smem, stream, map_w,
-                                                  map_x, bias, residual, out, ldo, M, N, K, mode, plan, status);
+                                                  map_x, bias, residual, out, ldo, M, N, K, mode, plan, parts, ldp, status);
     if (e != cudaSuccess) {
         mx_set_error("column gemm: launch failed: %s", cudaGetErrorString(e));
         return (int)e;
     }
+    if (plan.splits > 1 && finish)
+        return mx_add_parts(parts, ldp, plan.splits, bias, reinterpret_cast<float*>(out), ldo, M, N, stream);
     return MX_OK;
 }

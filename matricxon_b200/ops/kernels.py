@@ -115,21 +115,21 @@ def layernorm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, 
 
 def layernorm_sum(x: torch.Tensor, acc: torch.Tensor, col_bias: torch.Tensor | None, weight: torch.Tensor,
                   bias: torch.Tensor | None, eps: float, out: torch.Tensor) -> None:
-    """``x += acc + col_bias`` (the residual epilogue of a product whose float accumulator is ``acc``),
-    then ``out = LayerNorm(x)``, in one pass over the rows."""
+    """``x += acc + col_bias`` (the residual epilogue of a product whose float accumulator is ``acc``, or the sum of its
+    parts [parts, rows, columns]), then ``out = LayerNorm(x)``, in one pass over the rows."""
     _need(x, "x", torch.float32)
     _need(acc, "acc", torch.float32)
     _need(weight, "weight", torch.float32)
     _need(out, "out")
-    assert acc.shape == x.shape and out.shape == x.shape, (x.shape, acc.shape, out.shape)
+    assert acc.shape[-2:] == x.shape and acc.ndim <= 3 and out.shape == x.shape, (x.shape, acc.shape, out.shape)
     if col_bias is not None:
         _need(col_bias, "col_bias", torch.float32)
         assert col_bias.numel() == x.shape[1]
     if bias is not None:
         _need(bias, "bias", torch.float32)
-    check(library().mx_layernorm_sum(_ptr(x), _ptr(acc), _ptr(col_bias), _ptr(weight), _ptr(bias), _ptr(out),
-                                     dtype_code(out.dtype), x.shape[0], x.shape[1], float(eps), _stream()),
-          "layernorm_sum")
+    check(library().mx_layernorm_sum(_ptr(x), _ptr(acc), acc.shape[0] if acc.ndim == 3 else 1, _ptr(col_bias), _ptr(weight),
+                                     _ptr(bias), _ptr(out), dtype_code(out.dtype), x.shape[0], x.shape[1], float(eps),
+                                     _stream()), "layernorm_sum")
     _launched()
 
 
@@ -314,9 +314,48 @@ def gemm_columns(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None,
         assert tuple(residual.shape) == (m, n) and residual.stride(0) == out.stride(0)
     if status is None:
         status = default_status(a.device)
+    in_place = mode == EPILOGUE_RESIDUAL and residual is not None and residual.data_ptr() == out.data_ptr()
+    n_parts = columns_gemm_parts(m, n, k) if in_place else 1
+    parts = torch.empty((n_parts, m, (n + 3) // 4 * 4), dtype=torch.float32, device=a.device) if n_parts > 1 else None
     check(library().mx_gemm_columns(_ptr(a), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out),
-                                    dtype_code(out.dtype), m, n, k, a.stride(0), w.stride(0),
+                                    dtype_code(out.dtype), _ptr(parts), 1, m, n, k, a.stride(0), w.stride(0),
                                     out.stride(0), mode, _ptr(status), _stream()), "gemm_columns")
+    _launched(2 if n_parts > 1 else 1)
+
+
+def columns_gemm_parts(m: int, n: int, k: int) -> int:
+    """Parts of K that ``gemm_columns`` cuts a product into that is added to the stream in place (1: none)."""
+    return library().mx_gemm_columns_parts(m, n, k)
+
+
+def gemm_columns_in_parts(a: torch.Tensor, w: torch.Tensor, residual: torch.Tensor) -> torch.Tensor:
+    """The product whose sum with ``residual`` is asked for, left in its parts of K: [parts, M, N] float32 for
+    ``layernorm_sum`` or ``add_parts``. N is a multiple of 4, and ``columns_gemm_parts`` above 1."""
+    _need(a, "a", torch.bfloat16, contiguous=False)
+    _need(w, "w", torch.bfloat16)
+    _need(residual, "residual", torch.float32)
+    m, k = a.shape
+    n = w.shape[0]
+    n_parts = columns_gemm_parts(m, n, k)
+    assert w.shape[1] == k and tuple(residual.shape) == (m, n) and n % 4 == 0 and n_parts > 1, (a.shape, w.shape, n_parts)
+    parts = torch.empty((n_parts, m, n), dtype=torch.float32, device=a.device)
+    check(library().mx_gemm_columns(_ptr(a), _ptr(w), None, _ptr(residual), _ptr(residual), dtype_code(torch.float32),
+                                    _ptr(parts), 0, m, n, k, a.stride(0), w.stride(0), residual.stride(0), EPILOGUE_RESIDUAL,
+                                    _ptr(default_status(a.device)), _stream()), "gemm_columns")
+    _launched()
+    return parts
+
+
+def add_parts(parts: torch.Tensor, bias: torch.Tensor | None, out: torch.Tensor) -> None:
+    """``out += bias + parts[0] + parts[1] + ..``: what a product left in parts of K, added up in their order."""
+    _need(parts, "parts", torch.float32)
+    _need(out, "out", torch.float32)
+    n_parts, m, n = parts.shape
+    assert tuple(out.shape) == (m, n), (parts.shape, out.shape)
+    if bias is not None:
+        _need(bias, "bias", torch.float32)
+        assert bias.numel() == n
+    check(library().mx_add_parts(_ptr(parts), n, n_parts, _ptr(bias), _ptr(out), out.stride(0), m, n, _stream()), "add_parts")
     _launched()
 
 

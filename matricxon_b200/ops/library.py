@@ -30,7 +30,7 @@ _SIGNATURES: dict[str, tuple[list, object]] = {
     "mx_embed": ([P, P, I, P, I, I, I, F, P, P], I),
     "mx_softcap": ([P, L, F, P], I),
     "mx_layernorm": ([P, P, P, P, P, I, I, I, F, P], I),
-    "mx_layernorm_sum": ([P, P, P, P, P, P, I, I, I, F, P], I),
+    "mx_layernorm_sum": ([P, P, I, P, P, P, P, I, I, I, F, P], I),
     "mx_rope_kv_write": ([P, I, I, P, P, P, P, I, I, I, I, I, I, L, I, P, P], I),
     "mx_rope_kv_write_bias": ([P, I, I, P, P, P, P, I, I, I, I, I, I, L, I, P, P, P], I),
     "mx_epilogue": ([P, I, P, P, P, I, L, I, I, P], I),
@@ -45,7 +45,9 @@ _SIGNATURES: dict[str, tuple[list, object]] = {
     "mx_gemm_skinny_blocks": ([I, I, I], I),
     "mx_gemm_stream": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P, P], I),
     "mx_gemm_columns_pays": ([I, I, I], I),
-    "mx_gemm_columns": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P, P], I),
+    "mx_gemm_columns_parts": ([I, I, I], I),
+    "mx_gemm_columns": ([P, P, P, P, P, I, P, I, I, I, I, I, I, I, I, P, P], I),
+    "mx_add_parts": ([P, I, I, P, P, I, I, I, P], I),
     "mx_gemm_skinny": ([P, P, P, P, P, I, I, I, I, I, I, I, I, P], I),
     "mx_gemm_skinny_rope": ([P, P, P, P, I, I, I, I, I, P, P, P, P, L, I, I, I, I, P, P], I),
     "mx_attention_scratch_bytes": ([I, I, I, I], L),

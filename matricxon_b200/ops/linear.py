@@ -93,13 +93,24 @@ def _pick(x: torch.Tensor, weight: torch.Tensor, m: int, n: int) -> str:
 
 class PendingSum:
     """``residual + x @ W.T + bias`` not yet added up: the library's float product of a step with 17 or
-    more rows, handed to the norm that follows, which forms the sum on its way through the rows
-    (``kernels.layernorm_sum``) instead of an epilogue pass of its own. ``tensor()`` adds it up for
-    anybody else. ``acc`` None: only a vector (``bias``) is still to be added to every row."""
+    more rows, or the parts of K of a "columns" product, handed to the norm that follows, which forms the
+    sum on its way through the rows (``kernels.layernorm_sum``) instead of an epilogue pass of its own.
+    ``tensor()`` adds it up for anybody else. ``acc`` None: only a vector (``bias``) is still to be added to
+    every row; ``parts`` [parts, rows, columns] (or None): ``acc`` is their sum."""
 
-    def __init__(self, acc: torch.Tensor | None, bias: torch.Tensor | None, residual: torch.Tensor) -> None:
-        self.acc, self.bias, self.residual = acc, bias, residual
+    def __init__(self, acc: torch.Tensor | None, bias: torch.Tensor | None, residual: torch.Tensor,
+                 parts: torch.Tensor | None = None) -> None:
+        self._acc, self.bias, self.residual = acc, bias, residual
+        self.parts = parts
         self._done = False
+
+    @property
+    def acc(self) -> torch.Tensor | None:
+        """The product as one tensor (formed now if it was left in parts)."""
+        if self.parts is not None:
+            kernels.add_parts(self.parts[1:], None, self.parts[0])
+            self._acc, self.parts = self.parts[0], None
+        return self._acc
 
     @property
     def shape(self):
@@ -119,7 +130,10 @@ class PendingSum:
         return self.residual
 
     def tensor(self) -> torch.Tensor:
-        if not self._done and self.acc is None:
+        if not self._done and self.parts is not None:
+            kernels.add_parts(self.parts, self.bias, self.residual)
+            self._done = True
+        elif not self._done and self.acc is None:
             kernels.add_row(self.residual, self.bias)
         elif not self._done:
             kernels.epilogue(self.acc, self.bias, self.residual, self.residual, EPILOGUE_RESIDUAL)
@@ -141,8 +155,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, mod
     mode EPILOGUE_NONE / EPILOGUE_GELU / EPILOGUE_RELU2 (the square of relu) give the compute dtype; EPILOGUE_RESIDUAL
     (``residual + x @ W.T + bias``) and EPILOGUE_F32 give float32.
 
-    ``defer_sum`` (EPILOGUE_RESIDUAL into the residual itself): where the product is the library's, the
-    caller gets a ``PendingSum`` instead of the sum and hands it to a norm that adds as it reads.
+    ``defer_sum`` (EPILOGUE_RESIDUAL into the residual itself): where the product is the library's, or "columns" with K in
+    parts, the caller gets a ``PendingSum`` instead of the sum and hands it to a norm that adds as it reads.
     """
     m, n = x.shape[0], weight.shape[0]
     out_dtype = torch.float32 if mode in (EPILOGUE_RESIDUAL, EPILOGUE_F32) else x.dtype
@@ -158,6 +172,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, mod
         acc = _mm_f32(x, weight.t())
         if acc is not None:
             return PendingSum(acc, bias, residual)
+    if (defer_sum and backend == "columns" and mode == EPILOGUE_RESIDUAL and out is residual and residual is not None
+            and n % 4 == 0 and m > 0 and kernels.columns_gemm_parts(m, n, x.shape[1]) > 1):
+        return PendingSum(None, bias, residual, kernels.gemm_columns_in_parts(x, weight, residual))
     if backend == "library" and out is None and mode == EPILOGUE_NONE and bias is None and m > 0:
         return torch.mm(x, weight.t())        # nothing to add: the library's result is the result
     if out is None:

@@ -43,7 +43,8 @@ class LayerNorm(Norm):
         kernel forms the sum, writes it to the residual stream and normalises it. Returns (x, norm(x))."""
         x = pending.added_by_kernel()
         out = torch.empty(tuple(x.shape), dtype=self.runtime.dtype, device=x.device)
-        kernels.layernorm_sum(x, pending.acc, pending.bias, self.weight, self.bias, self.spec.eps, out)
+        acc = pending.parts if pending.parts is not None else pending.acc
+        kernels.layernorm_sum(x, acc, pending.bias, self.weight, self.bias, self.spec.eps, out)
         return x, out
 
 

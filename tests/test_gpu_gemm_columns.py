@@ -69,3 +69,61 @@ def test_nan_stays_in_its_row():
     bad = ~out.isfinite().all(dim=1)
     assert bad.nonzero().flatten().tolist() == [3, 5] and bool(out[3].isnan().all())
     assert torch.equal(out[5], w[:, 0].float().sign() * math.inf)
+
+
+@pytest.mark.parametrize("m,n,k_dim", [(257, 3072, 12288), (512, 3072, 12288), (600, 2048, 8192), (1024, 1024, 6144),
+                                       (2048, 1024, 6144)])
+def test_parts_of_k_are_added_in_their_order(m, n, k_dim):
+    """A product whose K is cut into parts gives the same bits every time, whoever adds the parts up."""
+    from matricxon_b200.ops import kernels as k
+    from matricxon_b200.ops.linear import PendingSum, linear
+
+    assert k.columns_gemm_parts(m, n, k_dim) > 1
+    torch.manual_seed(m)
+    a, w = torch.randn(m, k_dim, device=DEV).bfloat16(), (torch.randn(n, k_dim, device=DEV) / math.sqrt(k_dim)).bfloat16()
+    bias, residual = torch.randn(n, device=DEV), 100 * torch.randn(m, n, device=DEV)
+    weight, shift = torch.randn(n, device=DEV), torch.randn(n, device=DEV)
+
+    def product(**options):
+        x = residual.clone()
+        return linear(a, w, bias, k.EPILOGUE_RESIDUAL, residual=x, out=x, backend="columns", **options)
+
+    first = product()
+    for _ in range(12):
+        assert torch.equal(product(), first)
+    exact = residual.double() + a.double() @ w.double().T + bias.double()
+    # the cut-offs of the running sum, and eight roundings of sums of the stream's size
+    bound = (k_dim / 16 + 16) * 2.0 ** -23 * (a.double().abs() @ w.double().abs().T) + 8 * 2.0 ** -23 * (exact.abs() + residual.abs())
+    assert bool(((first.double() - exact).abs() <= bound).all())
+    pending = product(defer_sum=True)
+    assert isinstance(pending, PendingSum) and torch.equal(pending.tensor(), first) and torch.equal(pending.tensor(), first)
+    pending = product(defer_sum=True)
+    normed, alone = (torch.empty(m, n, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    x = pending.added_by_kernel()
+    k.layernorm_sum(x, pending.parts, pending.bias, weight, shift, 1e-5, normed)
+    k.layernorm(first, weight, shift, 1e-5, alone)
+    assert torch.equal(x, first) and torch.equal(normed, alone)
+    pending = product(defer_sum=True)                                      # for norms that take one tensor
+    assert bool(((pending.acc.double() - (exact - residual - bias)).abs() <= bound).all()) and pending.parts is None
+    assert bool(((pending.tensor().double() - exact).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("rows,columns,n_parts", [(1, 4, 2), (300, 3072, 3), (7, 8196, 8), (5, 30, 4), (3, 52000, 2)])
+def test_norm_of_parts(rows, columns, n_parts):
+    """Rows in registers, rows too long for them, rows that cannot be read 16 bytes at a time."""
+    from matricxon_b200.ops import kernels as k
+
+    parts, residual = torch.randn(n_parts, rows, columns, device=DEV), torch.randn(rows, columns, device=DEV)
+    bias, weight = torch.randn(columns, device=DEV), torch.randn(columns, device=DEV)
+    total = parts[0].clone()
+    for p in parts[1:]:
+        total += p
+    want = (total + bias) + residual
+    added = residual.clone()
+    k.add_parts(parts, bias, added)
+    assert torch.equal(added, want)
+    if columns <= 51200:
+        x, out, alone = residual.clone(), torch.empty_like(want), torch.empty_like(want)
+        k.layernorm_sum(x, parts, bias, weight, None, 1e-5, out)
+        k.layernorm(want, weight, None, 1e-5, alone)
+        assert torch.equal(x, want) and torch.equal(out, alone)
