@@ -216,6 +216,7 @@ gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             const int stride = shared ? ldp : ldo;
             for (int c = 0; c < tokens; c += 16) {
                 unsigned r[16];
+                __syncwarp();                           // lanes beyond N have gone past the stores
                 tmem_load16(from + (unsigned)c, r);
                 const size_t o = (size_t)(m0 + column + c) * stride + n;
                 if constexpr (F32) {
