@@ -74,7 +74,7 @@ struct MmaAttnParams {
     float cap_log2, cap_in;
     const float* sink;           // [heads] or null: exp(sink[h]) joins the softmax's denominator, with no value
     const float* distance;       // [2][heads] (r1, then r2) or null: scores lose r1 ln(1 + r2 (p - j))
-    int beside;                  // the next kernel starts beside this one and waits for nobody else (attention_tc.cu)
+    int beside;                  // the next kernel runs beside this one and takes what this one waited for (attention_tc.cu)
 };
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], unsigned a0, unsigned a1, unsigned a2,
@@ -264,7 +264,10 @@ attention_mma_kernel(const MmaAttnParams p) {
     const int q_len = p.cu_q[seq + 1] - q_start;
     const int ctx = p.context_lens[seq];
     const int n_rows = q_len * group;
-    if (tile_row0 >= n_rows) return;            // a padding sequence of a fixed-size batch
+    if (tile_row0 >= n_rows) {                  // a padding sequence of a fixed-size batch
+        if (p.beside) pdl_wait();               // a block that ends has let the next kernel start
+        return;
+    }
 
     if (tid == 0) {
 #pragma unroll
@@ -758,6 +761,26 @@ extern "C" int mx_attention_merge_bf16_sink(const float* part_o, const float* pa
                                             int out_stride, int n_tokens, int n_heads, int head_dim,
                                             int n_splits, const float* sink, cudaStream_t stream);
 
+namespace {
+// The launch that another kernel may run beside, if it is this thread's last one (mx_attention_beside_follows).
+thread_local struct {
+    unsigned long long launches;
+    const void *q, *cache, *cu_q, *context_lens, *out;
+    cudaStream_t stream;
+} g_beside = {};
+}  // namespace
+
+// Whether this thread's last launch is mx_paged_attention_mma with `beside`, of the same step's tensors on the same stream.
+// Holds once: what launches next is no longer beside it.
+bool mx_attention_beside_follows(const void* q, const void* cache, const void* cu_q, const void* context_lens, const void* out,
+                                 cudaStream_t stream) {
+    const bool follows = g_beside.launches != 0 && g_beside.launches == mx_launches() && g_beside.q == q && g_beside.cache == cache &&
+                         g_beside.cu_q == cu_q && g_beside.context_lens == context_lens && g_beside.out == out &&
+                         g_beside.stream == stream;
+    g_beside = {};
+    return follows;
+}
+
 // `narrow` != 0: every tile has at most 16 rows (decode tokens); the eight warps of a block
 // share them and take the key chunks in turn. Otherwise tiles are 64 rows, 16 per warp.
 extern "C" int mx_paged_attention_mma(const void* q, int q_stride, const void* cache,
@@ -780,6 +803,7 @@ extern "C" int mx_paged_attention_mma(const void* q, int q_stride, const void* c
     if (n_splits < 1 || n_splits > 65535) MX_REFUSE("attention: n_splits %d", n_splits);
     if (n_kv_heads > 65535) MX_REFUSE("attention: %d kv heads exceed the grid", n_kv_heads);
     if (n_splits > 1 && scratch == nullptr) MX_REFUSE("attention: split path without scratch memory");
+    if (beside && n_splits > 1) MX_REFUSE("attention that another kernel runs beside takes no key splits");
     MmaAttnParams p;
     p.q = (const __nv_bfloat16*)q; p.cache = (const __nv_bfloat16*)cache; p.out = (__nv_bfloat16*)out;
     p.part_o = scratch;
@@ -800,6 +824,7 @@ extern "C" int mx_paged_attention_mma(const void* q, int q_stride, const void* c
     int rc;
     if (head_dim == 64) rc = narrow ? launch_mma<64, true>(p, stream) : launch_mma<64, false>(p, stream);
     else rc = narrow ? launch_mma<128, true>(p, stream) : launch_mma<128, false>(p, stream);
+    if (rc == MX_OK && beside) g_beside = {mx_launches(), q, cache, cu_q, context_lens, out, stream};
     if (rc != MX_OK || n_splits == 1) return rc;
     return mx_attention_merge_bf16_sink(p.part_o, p.part_ml, out, out_stride, n_tokens, n_heads, head_dim,
                                         n_splits, sink, stream);

@@ -252,7 +252,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     // tiles start in the order of their list, which puts the ones with the most keys first, all heads of a tile side by
     // side (2,048 tokens, us in the list's order and from its end: 24 query heads on 2 KV heads 53 and 59, 16 on 16 32 and 41)
-    // (beside another kernel nothing is waited for here: what earlier kernels wrote is in memory, also for the copies below)
+    // Beside the decoding requests' attention (mx_paged_attention_mma, `beside`) nothing is waited for here. What this kernel
+    // reads was written by the kernels before that one. Every block of that one has waited for their end, at which what they
+    // wrote is in memory for the whole device, before it let this kernel start; this kernel's blocks begin after that, with
+    // nothing of it in their L1, and the copies below read L2 (the fence is for them). That the launch directly before is
+    // that kernel, on this step's tensors, is checked when this one is launched.
     asm volatile("fence.proxy.async.global;\n" ::: "memory");
     const int tile = (int)(blockIdx.x / (unsigned)p.n_kv_heads);
     const int kh = (int)(blockIdx.x % (unsigned)p.n_kv_heads);
@@ -261,7 +265,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     const int q_len = p.cu_q[seq + 1] - q_start;
     const int ctx = p.context_lens[seq];
     const int n_tok = min(p.tokens_per_tile, q_len - tok0);
-    if (n_tok <= 0) return;                                         // nothing was allocated yet
+    if (n_tok <= 0) {                                               // nothing was allocated yet
+        pdl_wait();
+        return;
+    }
     const int hi_tile = ctx + tok0 + n_tok - 1;
     const int lo_tile = first_visible_key(ctx + tok0, p.window);
     // the tile's chunks of 128 keys, and this block's share of them when the keys are split (few tiles, a
@@ -722,6 +729,8 @@ int at_make_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* 
 extern "C" int mx_attention_merge_bf16_sink(const float* part_o, const float* part_ml, void* out, int out_stride,
                                             int n_tokens, int n_heads, int head_dim, int n_splits, const float* sink,
                                             cudaStream_t stream);
+bool mx_attention_beside_follows(const void* q, const void* cache, const void* cu_q, const void* context_lens, const void* out,
+                                 cudaStream_t stream);          // attention_mma.cu
 
 // n_splits > 1: every tile's keys are shared out between n_splits blocks, whose partial results go to
 // `scratch` ((tokens x heads x splits) x (128 + 2) floats) and are merged by mx_attention_merge_bf16.
@@ -800,6 +809,8 @@ extern "C" int mx_paged_attention_tc_split(const void* q, int q_stride, const vo
     if ((long long)n_tiles * n_kv_heads > 0x7fffffffLL) MX_REFUSE("tcgen05 attention: %d tiles exceed the grid", n_tiles);
     const dim3 grid((unsigned)(n_tiles * n_kv_heads), 1, n_splits);
     if (beside) {
+        if (!mx_attention_beside_follows(q, cache, cu_q, context_lens, out, stream))
+            MX_REFUSE("tcgen05 attention beside another kernel: the launch before is not that kernel, of the same step");
         // The decoding requests' attention, launched just before, lets this kernel start once each of its blocks has seen
         // the end of what both need (attention_mma.cu): the prompt's tiles then take the SMs that it leaves free, and those
         // that its short requests give back. They wait for it only before they end. 31 requests of up to 6,000 tokens and a

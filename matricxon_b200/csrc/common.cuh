@@ -33,7 +33,12 @@ void mx_set_error(const char* fmt, ...);
         return MX_ERR_UNSUPPORTED;  \
     } while (0)
 
+// Every launch of this library goes on record, by thread: mx_launches() changes whenever the calling thread launches.
+void mx_count_launch();
+unsigned long long mx_launches();
+
 static inline int mx_launch_status() {
+    mx_count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         mx_set_error("CUDA launch failed: %s", cudaGetErrorString(e));
@@ -83,6 +88,7 @@ static inline cudaError_t mx_launch_chained(void (*kernel)(KArgs...), dim3 grid,
     attribute[0].val.programmaticStreamSerializationAllowed = mx_chained_launch_enabled() ? 1 : 0;
     config.attrs = attribute;
     config.numAttrs = 1;
+    mx_count_launch();
     return cudaLaunchKernelEx(&config, kernel, KArgs(args)...);
 }
 

@@ -31,6 +31,10 @@ bool mx_chained_launch_enabled() {
     return forced >= 0 ? forced == 1 : g_chained_launch == 1;
 }
 
+static thread_local unsigned long long g_launches = 0;
+void mx_count_launch() { ++g_launches; }
+unsigned long long mx_launches() { return g_launches; }
+
 void mx_set_error(const char* fmt, ...) {
     va_list ap;
     va_start(ap, fmt);

@@ -694,6 +694,7 @@ extern "C" int mx_gemm_f32_split(const float* A, const float* W, const float* bi
         cudaLaunchConfig_t config;
         cudaLaunchAttribute attribute[2];
         fs_config(config, attribute, (int)blocks, plan.splits, smem, stream);
+        mx_count_launch();
         e = cudaLaunchKernelEx(&config, gemm_f32_split_kernel, map_w, map_x, A, lda, W, ldw, bias, residual, out, ldo, M, N,
                                K, mode, (const FsPlan)plan, status);
     }

@@ -367,6 +367,7 @@ extern "C" int mx_gemm_skinny(const void* x, const void* W, const float* bias, c
         attribute[1].val.programmaticStreamSerializationAllowed = mx_chained_launch_enabled() ? 1 : 0;
         config.attrs = attribute;
         config.numAttrs = 2;
+        mx_count_launch();
         const cudaError_t e = cudaLaunchKernelEx(&config, kernel, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)W,
                                                  ldw, bias, residual, out, ldo, M, N, K, mode, none);
         if (e != cudaSuccess) {

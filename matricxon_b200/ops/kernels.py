@@ -585,7 +585,8 @@ def paged_attention_tc(q: torch.Tensor, q_stride: int, cache: torch.Tensor, bloc
     (``attention_tile_lists(..., token_tiles=True)``); ``q`` holds the step's rows, query head h
     at column h * head_dim. ``n_splits`` > 1 shares every tile's keys out between that many blocks
     (few tiles, long contexts); ``scratch`` (float32, ``attention_scratch_bytes``) takes their parts. ``beside``: the
-    launch before this one is ``paged_attention_mma(..., beside=True)`` of the same step, and both run at a time."""
+    launch before this one is ``paged_attention_mma(..., beside=True)`` of the same step, and both run at a time; after
+    any other launch of the library this is refused."""
     _need(q, "q", torch.bfloat16, contiguous=False)
     _need(cache, "cache", torch.bfloat16)
     for name, tensor in (("block_tables", block_tables), ("cu_q", cu_q),
