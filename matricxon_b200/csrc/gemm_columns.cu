@@ -256,24 +256,24 @@ gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     }
 }
 
-// Pairs of SMs that run at a time (0: the kernel cannot run).
+// Pairs of SMs that run at a time (0: the kernel cannot run), looked up by the first call while others wait for it.
 int cl_pairs() {
-    static int count = -1;
-    if (count < 0) {
-        count = 0;
+    static const int count = [] {
+        int clusters = 0;
         if (cudaFuncSetAttribute(gemm_columns_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM) == cudaSuccess &&
             cudaFuncSetAttribute(gemm_columns_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM) == cudaSuccess) {
-            int device = 0, sms = 0, clusters = 0;
+            int device = 0, sms = 0;
             cudaGetDevice(&device);
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
             cudaLaunchConfig_t config = {};
             config.gridDim = dim3(2 * max(1, sms / 2));
             config.blockDim = dim3(CL_THREADS);
             config.dynamicSmemBytes = CL_SMEM;
-            if (cudaOccupancyMaxActiveClusters(&clusters, gemm_columns_kernel<true>, &config) == cudaSuccess) count = clusters;
+            if (cudaOccupancyMaxActiveClusters(&clusters, gemm_columns_kernel<true>, &config) != cudaSuccess) clusters = 0;
         }
         cudaGetLastError();
-    }
+        return clusters;
+    }();
     return count;
 }
 

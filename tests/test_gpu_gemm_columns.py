@@ -2,6 +2,9 @@
 parts of K, every epilogue, more items than pairs, and what is not finite."""
 
 import math
+import os
+import subprocess
+import sys
 
 import pytest
 
@@ -127,3 +130,35 @@ def test_norm_of_parts(rows, columns, n_parts):
         k.layernorm_sum(x, parts, bias, weight, None, 1e-5, out)
         k.layernorm(want, weight, None, 1e-5, alone)
         assert torch.equal(x, want) and torch.equal(out, alone)
+
+
+FIRST_CALLS = """
+import sys, threading
+sys.path.insert(0, sys.argv[1])
+import torch
+from matricxon_b200.ops import kernels as k
+a, w = torch.randn(300, 512, device="cuda").bfloat16(), torch.randn(1024, 512, device="cuda").bfloat16()
+outs = [torch.empty(300, 1024, device="cuda") for _ in range(8)]
+k.default_status(a.device)
+torch.cuda.synchronize()
+barrier, failed = threading.Barrier(len(outs)), []
+def call(out):
+    barrier.wait()
+    try:
+        k.gemm_columns(a, w, None, None, out, k.EPILOGUE_F32)
+    except Exception as error:
+        failed.append(error)
+threads = [threading.Thread(target=call, args=(out,)) for out in outs]
+for t in threads: t.start()
+for t in threads: t.join()
+torch.cuda.synchronize()
+assert not failed, failed
+assert all(torch.equal(out, outs[0]) for out in outs)
+"""
+
+
+def test_first_calls_from_several_threads():
+    """What the first call of a process looks up (pairs of SMs, shared memory) is there for all that come meanwhile."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", FIRST_CALLS, root], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
