@@ -9,7 +9,10 @@
 // piece). Root mean square error against 64 bits, of the result's: 1.1e-7 to 1.9e-7 for K = 3,072 (by the shares of K; the FP32
 // cores 5.0e-7), 1.8e-7 to 3.6e-7 for K = 12,288 (1.0e-6).
 // A result that is not finite (an operand that is not, an overflow on the way, a float above bfloat16's largest) is formed
-// again from the operands by plain multiply-adds, which decide what it is. The reference runs these products through
+// again from the operands by plain multiply-adds, which decide what it is, unless its row of A holds a NaN, which decides it:
+// a warp looks at the row first (one such row among 4 of 3,072 x 12,288 took 558 us as chains and takes 40, the product 40;
+// 389 of 389 rows of 12,288 x 3,072 61,200 and 183, the product 169). An infinity or an overflow in a row still costs the
+// chains (245 us at 4 rows of 12,288, 501 at 389 of 3,072). The reference runs these products through
 // nn.Linear (app/architectures/qwen_layers.py:50-53, app/architectures/starcoder2_layers.py:19-23).
 //
 // Weight rows are the tensor cores' 128 rows, tokens the columns (up to 208). The weights come as floats by TMA, since a
@@ -156,14 +159,41 @@ __device__ __forceinline__ void umma_bf16_ts_elect(unsigned tmem_acc, unsigned t
         : "memory");
 }
 
-// What the FP32 cores give for one result, in the order of gemm_simt.cu.
+// ---- results that are not finite
+// Whether a row of A holds a NaN (its results are then NaN): a whole warp looks at it.
+__device__ __noinline__ bool row_has_nan(const float* a, int K) {
+    const int lane = threadIdx.x & 31;
+    bool found = false;
+    for (int k0 = 0; k0 < K; k0 += 16 * 32) {
+        float4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k = k0 + 4 * (i * 32 + lane);
+            v[i] = k < K ? *reinterpret_cast<const float4*>(a + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) found = found || isnan(v[i].x) || isnan(v[i].y) || isnan(v[i].z) || isnan(v[i].w);
+        if (__any_sync(0xffffffffu, found)) return true;
+    }
+    return false;
+}
+
+// What the FP32 cores give for one result, in the order of gemm_simt.cu: its four chains side by side, 16 bytes at a time.
 __device__ __noinline__ float plain_product(const float* a, const float* w, int K) {
-    const int piece = f32_piece(K);
-    float total[F32_PIECES];
-    for (int i = 0; i < F32_PIECES; ++i) {
-        float p = 0.f;
-        for (int k = min(i * piece, K); k < min((i + 1) * piece, K); ++k) p = fmaf(a[k], w[k], p);
-        total[i] = p;
+    const int piece = f32_piece(K);                     // a multiple of 32, as K is one of 4
+    float total[F32_PIECES] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+    for (int k = 0; k < piece; k += 4) {
+        float4 x[F32_PIECES], y[F32_PIECES];
+#pragma unroll
+        for (int i = 0; i < F32_PIECES; ++i) {
+            const bool in = i * piece + k < K;
+            x[i] = in ? *reinterpret_cast<const float4*>(a + i * piece + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            y[i] = in ? *reinterpret_cast<const float4*>(w + i * piece + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < F32_PIECES; ++i)
+            total[i] = fmaf(x[i].w, y[i].w, fmaf(x[i].z, y[i].z, fmaf(x[i].y, y[i].y, fmaf(x[i].x, y[i].x, total[i]))));
     }
     return (total[0] + total[1]) + (total[2] + total[3]);
 }
@@ -370,14 +400,14 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         float b[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) b[e] = bias != nullptr && n + e < N ? bias[n + e] : 0.f;
-        // four tokens at a time, so that their reads are out together
-        for (int j0 = rank + plan.splits * warp; j0 < plan.tokens && n < N; j0 += plan.splits * FS_ADDERS * 4) {
+        // four tokens at a time, so that their reads are out together (lanes beyond N go along)
+        for (int j0 = rank + plan.splits * warp; j0 < plan.tokens; j0 += plan.splits * FS_ADDERS * 4) {
             float4 v[4], res[4];
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 v[t] = res[t] = make_float4(0.f, 0.f, 0.f, 0.f);
                 const int j = j0 + t * plan.splits * FS_ADDERS;
-                if (mode == MX_MODE_RESIDUAL && j < plan.tokens && m0 + j < M) {
+                if (mode == MX_MODE_RESIDUAL && j < plan.tokens && m0 + j < M && n < N) {
                     const float* from = residual + (size_t)(m0 + j) * ldo + n;
                     if (wide) {
                         res[t] = *reinterpret_cast<const float4*>(from);
@@ -407,9 +437,13 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 if (j >= plan.tokens || m >= M) break;
                 float y[4] = {v[t].x, v[t].y, v[t].z, v[t].w};
                 const float z[4] = {res[t].x, res[t].y, res[t].z, res[t].w};
-                if (!isfinite(y[0]) || !isfinite(y[1]) || !isfinite(y[2]) || !isfinite(y[3])) {
+                const bool finite = n >= N || (isfinite(y[0]) && isfinite(y[1]) && isfinite(y[2]) && isfinite(y[3]));
+                if (!__all_sync(0xffffffffu, finite)) {
+                    const bool nan = row_has_nan(A + (size_t)m * lda, K);
+#pragma unroll
                     for (int e = 0; e < 4; ++e)
-                        if (!isfinite(y[e]) && n + e < N) y[e] = plain_product(A + (size_t)m * lda, W + (size_t)(n + e) * ldw, K);
+                        if (!isfinite(y[e]) && n + e < N)
+                            y[e] = nan ? NAN : plain_product(A + (size_t)m * lda, W + (size_t)(n + e) * ldw, K);
                 }
                 float* to = out + (size_t)m * ldo + n;
 #pragma unroll
@@ -533,11 +567,18 @@ gemm_f32_skinny_kernel(const float* __restrict__ A, int lda, const float* __rest
     for (int i = 0; i < 4; ++i) sums[warp][2 * t + (i & 1)][g + 8 * (i >> 1)] = acc[i];
     __syncthreads();
     const int f = threadIdx.x % FK_ROWS, m = threadIdx.x / FK_ROWS, n = n0 + f;
-    if (m >= M || m >= FK_TOKENS || n >= N) return;
+    if (warp >= FK_TOKENS / 2) return;                  // a warp has the 16 columns of two tokens
+    const bool mine = m < M && n < N;
     float v = 0.f;
 #pragma unroll
     for (int w = 0; w < FK_WARPS; ++w) v += sums[w][m][f];
-    if (!isfinite(v)) v = plain_product(A + (size_t)m * lda, W + (size_t)n * ldw, K);
+    for (int half = 0; half < 2; ++half) {
+        const bool again = mine && (lane >> 4) == half && !isfinite(v);
+        if (!__any_sync(0xffffffffu, again)) continue;
+        const bool nan = row_has_nan(A + (size_t)(2 * warp + half) * lda, K);
+        if (again) v = nan ? NAN : plain_product(A + (size_t)m * lda, W + (size_t)n * ldw, K);
+    }
+    if (!mine) return;
     v = mode_activation(v + (bias != nullptr ? bias[n] : 0.f), mode);
     const size_t o = (size_t)m * ldo + n;
     if (mode == MX_MODE_RESIDUAL) v += residual[o];

@@ -86,3 +86,46 @@ def test_the_engine_takes_it_for_many_rows():
     assert chosen_backend(torch.empty(200, 512, device=DEV), w) == "split"
     assert chosen_backend(torch.empty(200, 512, device=DEV), w, "simt") == "simt"
     assert chosen_backend(torch.empty(200, 513, device=DEV)[:, 1:], w) == "simt"      # cannot be read 16 bytes at a time
+
+
+@pytest.mark.parametrize("m", [3, 8, 20, 300])
+def test_rows_that_are_not_finite_cost_the_others_little(m):
+    """Their results are what the FP32 cores give, and a NaN is found by a look at its row: not a chain of K multiply-adds for
+    every column, which made a step with one such row some ten times as long."""
+    from matricxon_b200.ops import kernels as k
+
+    n, k_dim = 2052, 4096
+    w = torch.randn(n, k_dim, device=DEV)
+    clean = torch.randn(m, k_dim, device=DEV)
+    with_nan, every, mixed = clean.clone(), clean.clone(), clean.clone()
+    with_nan[m - 1, k_dim - 1] = math.nan
+    every[:, 77] = math.nan
+    mixed[0, 9], mixed[1, 10], mixed[2, 100] = math.inf, -math.inf, 3.4e38
+    mixed[2] *= 1e-3
+    mixed[2, 100] = 3.4e38
+    out, plain = torch.empty(m, n, device=DEV), torch.empty(m, n, device=DEV)
+
+    def micros(a):
+        best = math.inf
+        for _ in range(6):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for _ in range(4):
+                k.gemm_f32_split(a, w, None, None, out, k.EPILOGUE_F32)
+            end.record()
+            end.synchronize()
+            best = min(best, start.elapsed_time(end) * 250)
+        return best
+
+    for a in (with_nan, every, mixed):
+        k.gemm_f32_split(a, w, None, None, out, k.EPILOGUE_F32)
+        k.gemm_simt(a, w, None, None, plain, k.EPILOGUE_F32)
+        odd = ~plain.isfinite()
+        assert bool((~out[odd].isfinite()).all()) and torch.equal(out[odd].isnan(), plain[odd].isnan())
+        assert bool((out[odd][~plain[odd].isnan()] == plain[odd][~plain[odd].isnan()]).all())
+        size = a.double().abs() @ w.double().abs().T
+        good = plain.isfinite()
+        assert bool(((out.double() - plain.double()).abs() <= (2.0 ** -24 + k_dim * 2.0 ** -24) * size)[good].all())
+    usual = micros(clean)
+    # a look at 16 KB of a row, and (every row) at 208 of them in eight warps; plain chains took 10 and 300 times as long
+    assert micros(with_nan) <= 2 * usual + 20 and micros(every) <= 8 * usual + 20
