@@ -675,6 +675,12 @@ bool sixteen_keys_a_warp(const AttnParams& p) {
            (reinterpret_cast<uintptr_t>(p.q) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.cache) & 31) == 0;
 }
 
+// Query heads of a block of the float kernel: up to six, dealt out evenly.
+int f32_heads(int group) {
+    const int parts = (group + 5) / 6;
+    return (group + parts - 1) / parts <= 4 ? 4 : 6;
+}
+
 template <typename T, int HD_SLOTS>
 int launch_attention(const AttnParams& p, int n_tokens, cudaStream_t stream) {
     const size_t smem = attention_smem_bytes<T>(p.head_dim);
@@ -688,8 +694,7 @@ int launch_attention(const AttnParams& p, int n_tokens, cudaStream_t stream) {
     dim3 grid(n_tokens, p.n_kv_heads * n_hgroups, p.n_splits);
     int rc;
     if (sixteen_keys_a_warp<T>(p)) {
-        const int parts = (group + 5) / 6, heads = (group + parts - 1) / parts;         // of a block, evenly dealt
-        rc = heads <= 4 ? launch_attention_f32<4>(p, n_tokens, stream) : launch_attention_f32<6>(p, n_tokens, stream);
+        rc = f32_heads(group) == 4 ? launch_attention_f32<4>(p, n_tokens, stream) : launch_attention_f32<6>(p, n_tokens, stream);
     } else {
         paged_attention_kernel<T, HD_SLOTS><<<grid, ATT_THREADS, smem, stream>>>(p);
         rc = mx_launch_status();
@@ -705,6 +710,16 @@ int launch_attention(const AttnParams& p, int n_tokens, cudaStream_t stream) {
 extern "C" long long mx_attention_scratch_bytes(int n_tokens, int n_heads, int head_dim, int n_splits) {
     if (n_splits <= 1) return 0;
     return (long long)n_tokens * n_heads * n_splits * (head_dim + 2) * (long long)sizeof(float);
+}
+
+// Blocks that mx_paged_attention deals the `group` query heads of a KV head out to, a token and key share each (the host sizes
+// the shares by them).
+extern "C" int mx_paged_attention_head_blocks(const void* q, int dtype, int q_stride, const void* cache, int page_size,
+                                              int head_dim, int group) {
+    AttnParams p = {};
+    p.q = q; p.q_stride = q_stride; p.cache = cache; p.page_size = page_size; p.head_dim = head_dim;
+    const int heads = dtype == MX_DTYPE_F32 && sixteen_keys_a_warp<float>(p) ? f32_heads(group) : GH;
+    return (group + heads - 1) / heads;
 }
 
 extern "C" int mx_paged_attention(const void* q, int dtype, int q_stride, const void* cache,

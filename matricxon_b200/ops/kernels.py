@@ -494,6 +494,11 @@ def attention_scratch_bytes(n_tokens: int, n_heads: int, head_dim: int, n_splits
     return int(library().mx_attention_scratch_bytes(n_tokens, n_heads, head_dim, n_splits))
 
 
+def attention_head_blocks(q: torch.Tensor, q_stride: int, cache: torch.Tensor, page_size: int, head_dim: int, group: int) -> int:
+    """Blocks of ``paged_attention`` that share the ``group`` query heads of a KV head, a token and key share each."""
+    return library().mx_paged_attention_head_blocks(_ptr(q), dtype_code(q.dtype), q_stride, _ptr(cache), page_size, head_dim, group)
+
+
 def paged_attention(q: torch.Tensor, q_stride: int, cache: torch.Tensor, block_tables: torch.Tensor,
                     tok_seq: torch.Tensor, positions: torch.Tensor, n_tokens: int, n_heads: int,
                     n_kv_heads: int, head_dim: int, window: int | None, scale: float,

@@ -54,6 +54,7 @@ _SIGNATURES: dict[str, tuple[list, object]] = {
     "mx_paged_attention_mma": ([P, I, P, L, I, P, I, P, P, P, I, I, I, I, I, I, I, F, P, I, I, P, P, F, P, I, P, I, P], I),
     "mx_paged_attention_tc": ([P, I, P, L, I, P, I, P, P, P, I, I, I, I, I, I, F, P, I, P, P], I),
     "mx_paged_attention_tc_split": ([P, I, P, L, I, P, I, P, P, P, I, I, I, I, I, I, F, P, I, I, P, P, F, P, I, P, I, P], I),
+    "mx_paged_attention_head_blocks": ([P, I, I, P, I, I, I], I),
     "mx_paged_attention": ([P, I, I, P, L, I, P, I, P, P, I, I, I, I, I, F, P, I, I, P, P, F, P, I, P, P], I),
     "mx_rmsnorm": ([P, P, P, F, P, I, I, I, F, L, P], I),
     "mx_add_row": ([P, P, I, I, P], I),
