@@ -604,6 +604,11 @@ void fs_config(cudaLaunchConfig_t& config, cudaLaunchAttribute (&attribute)[2], 
     config.numAttrs = 2;
 }
 
+// Lets the kernel use its shared memory on the current device.
+bool fs_ready() {
+    return cudaFuncSetAttribute(gemm_f32_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FS_SMEM) == cudaSuccess;
+}
+
 // Clusters of `splits` blocks that run at a time: what the device's groups of SMs leave room for.
 int fs_clusters(int splits) {
     static int known[FS_MAX_SPLITS + 1];                // the same on every GPU this library is built for
@@ -613,7 +618,7 @@ int fs_clusters(int splits) {
         fs_config(config, attribute, splits * 148, splits, FS_SMEM, nullptr);
         config.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, gemm_f32_split_kernel, &config) != cudaSuccess) {
+        if (!fs_ready() || cudaOccupancyMaxActiveClusters(&n, gemm_f32_split_kernel, &config) != cudaSuccess) {
             cudaGetLastError();
             n = 148 / splits;
         }
@@ -676,9 +681,10 @@ extern "C" int mx_gemm_f32_split_pays(int M, int N, int K) {
     return K >= (M <= 8 ? 512 : M <= 16 ? 2048 : M <= 32 ? 1024 : 512);
 }
 
-// Bytes of scratch that a product needs (0: none): the parts of A where a tile has more tokens than are split in passing.
+// Bytes of scratch that a product needs (0: none, and it is one launch instead of two): the parts of A where a tile has more
+// tokens than are split in passing.
 extern "C" long long mx_gemm_f32_split_scratch(int M, int N, int K) {
-    if (M <= FS_INLINE_TOKENS || N <= 0 || K <= 0) return 0;
+    if (M <= FS_INLINE_TOKENS || N <= 0 || K <= 0 || fs_plan(M, N, K).tokens <= FS_INLINE_TOKENS) return 0;
     return 3LL * M * ((K + 7) / 8 * 8) * 2;
 }
 
@@ -705,12 +711,7 @@ extern "C" int mx_gemm_f32_split(const float* A, const float* W, const float* bi
         }
         return MX_OK;
     }
-    static bool attribute_set = false;
-    if (!attribute_set) {
-        if (cudaFuncSetAttribute(gemm_f32_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FS_SMEM) != cudaSuccess)
-            MX_REFUSE("split gemm: cannot reserve %d bytes of shared memory", FS_SMEM);
-        attribute_set = true;
-    }
+    if (!fs_ready()) MX_REFUSE("split gemm: cannot reserve %d bytes of shared memory", FS_SMEM);
     FsPlan plan = fs_plan(M, N, K);
     const size_t smem = fs_stages(plan);
     const long long blocks = (long long)((N + FS_ROWS - 1) / FS_ROWS) * plan.token_tiles * plan.splits;

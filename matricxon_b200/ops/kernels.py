@@ -239,7 +239,7 @@ def gemm_f32_split(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None,
     check(library().mx_gemm_f32_split(_ptr(a), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), _ptr(scratch), m, n, k,
                                       a.stride(0), w.stride(0), out.stride(0), mode, _ptr(status), _stream()),
           "gemm_f32_split")
-    _launched()
+    _launched(2 if need else 1)
 
 
 _default_status: dict[int, torch.Tensor] = {}

@@ -129,3 +129,25 @@ def test_rows_that_are_not_finite_cost_the_others_little(m):
     usual = micros(clean)
     # a look at 16 KB of a row, and (every row) at 208 of them in eight warps; plain chains took 10 and 300 times as long
     assert micros(with_nan) <= 2 * usual + 20 and micros(every) <= 8 * usual + 20
+
+
+@pytest.mark.parametrize("m,n,twice", [(3, 300, False), (64, 300, False), (65, 300, None), (96, 300, None), (130, 1000, None),
+                                       (300, 300, None), (389, 12288, True)])
+def test_launches_are_counted(m, n, twice):
+    """Tiles of more than 64 tokens have them split by a kernel of its own, into scratch memory; others need neither (None:
+    whichever the plan takes)."""
+    from torch.profiler import ProfilerActivity, profile
+
+    from matricxon_b200.ops import kernels as k
+    from matricxon_b200.ops.library import library
+
+    a, w, out = torch.randn(m, 512, device=DEV), torch.randn(n, 512, device=DEV), torch.empty(m, n, device=DEV)
+    k.gemm_f32_split(a, w, None, None, out, k.EPILOGUE_F32)
+    torch.cuda.synchronize()
+    before = k.launch_count
+    with profile(activities=[ProfilerActivity.CUDA]) as seen:
+        k.gemm_f32_split(a, w, None, None, out, k.EPILOGUE_F32)
+        torch.cuda.synchronize()
+    kernels = sum(e.count for e in seen.key_averages() if "f32_split" in e.key or "f32_skinny" in e.key)
+    assert k.launch_count - before == kernels == 1 + (library().mx_gemm_f32_split_scratch(m, n, 512) > 0)
+    assert twice is None or kernels == 1 + twice
