@@ -203,8 +203,9 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None,
 
 
 def split_gemm_supported(a: torch.Tensor, w: torch.Tensor) -> bool:
+    # rows that lie in one another (a row expanded to several) are no tensor that TMA describes
     return (a.dtype == torch.float32 and w.dtype == torch.float32 and a.shape[1] % 4 == 0 and a.stride(1) == 1
-            and a.stride(0) % 4 == 0 and w.is_contiguous() and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+            and a.stride(0) % 4 == 0 and (a.shape[0] <= 1 or a.stride(0) >= a.shape[1]) and w.is_contiguous() and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def split_gemm_pays(m: int, n: int, k: int) -> bool:

@@ -13,3 +13,19 @@ def test_shortest_k(m, n, least):
     assert pays(m, n, least) and (least == 0 or not pays(m, n, least - 4))
     # a low-rank factor of a prompt stays with the general kernel, and so does a K whose fourth piece would be empty
     assert not pays(389, 2048, 16) and not pays(389, 2048, 160) and pays(389, 2048, 192)
+
+
+def test_rows_that_lie_in_one_another_stay_on_the_fp32_cores():
+    import torch
+    from matricxon_b200.ops.linear import chosen_backend
+
+    def at(make, m=40):
+        memory = torch.zeros(200 * 1028 + 8)
+        memory = memory[-(memory.data_ptr() // 4) % 4:]
+        return chosen_backend(make(memory, m), torch.zeros(512, 1024))
+
+    assert at(lambda x, m: x[:m * 1024].view(m, 1024)) == "split"
+    assert at(lambda x, m: x.as_strided((m, 1024), (1028, 1))) == "split"
+    assert at(lambda x, m: x[:1024].expand(m, 1024)) == "simt"              # one row for all
+    assert at(lambda x, m: x.as_strided((m, 1024), (4, 1))) == "simt"       # windows that slide by four numbers
+    assert at(lambda x, m: x.as_strided((m, 1024), (1026, 1))) == "simt"
