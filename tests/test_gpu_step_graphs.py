@@ -96,3 +96,82 @@ def test_graphs_of_shapes_are_bounded_and_the_oldest_goes():
         assert len(runner._shape_graphs) <= 2
     runner.check_status()
     assert [key[0][0] for key in runner._shape_graphs] == [7, 5]
+
+
+def large(kind, dtype):
+    """(core that captures, core that does not, vocabulary): layers wide enough for the kernels of real sizes (heads of 128 on
+    tcgen05, products with the tokens as columns, recurrences over groups and chunks), so that a captured step chains them."""
+    from matricxon_b200.engine.core import EngineCore, model_from_tensors
+
+    store = torch.float32 if dtype == "float32" else torch.bfloat16
+    if kind == "starcoder2":
+        from test_gpu_real_sizes import COMMON, make_material
+
+        raw = dict(COMMON, hidden_size=1024, num_attention_heads=8, num_key_value_heads=2, intermediate_size=8192,
+                   vocab_size=2048, rope_theta=10000.0, tie_word_embeddings=False, sliding_window=400)
+        config, tensors, _, _ = make_material(raw)
+        vocab = 2048
+    else:
+        import palelix_configs as p
+
+        raw = p.model(1024, 512, [
+            p.parallel((8, 2, 128, 128, 0.08, (64, 10000.0)), (8, 8, 128, 128, 4), 1.0, 1.0, mlp=p.dense(8192)),
+            p.lightning(8, 128, 128, [1 - 2.0 ** (-5 - i / 3) for i in range(8)], mlp=p.dense(8192)),
+            p.delta(8, 4, 128, 128, 4, mlp=p.dense(8192))])
+        tensors = p.draw(raw, 5, store)
+        config, vocab = p.config_of(raw, tensors), 512
+    cores = []
+    for use_graphs in (True, False):
+        model = model_from_tensors(config, {k: v.to(store) for k, v in tensors.items()}, dtype=dtype, device=DEV)
+        cores.append(EngineCore(model, max_cache_tokens=8192, max_requests=8, poison_cache=True, use_graphs=use_graphs))
+    return *cores, vocab
+
+
+@pytest.mark.parametrize("kind,dtype", [("starcoder2", "bfloat16"), ("starcoder2", "float32"), ("palelix", "bfloat16")])
+def test_captured_mixed_steps_chain_the_kernels_of_real_sizes(kind, dtype, monkeypatch):
+    """Three decoding requests beside portions of 300 tokens: eager, captured and replayed steps, which start each kernel while
+    the one before it drains (the two attention kernels at a time), give the logits of steps that do not."""
+    from matricxon_b200.engine.step import StepEntry
+    from matricxon_b200.ops import kernels
+
+    captured, eager, vocab = large(kind, dtype)
+    called = {}
+    for name in ("gemm_columns", "gemm_columns_in_parts", "gemm_f32_split", "paged_attention_tc"):
+        def counted(*args, _call=getattr(kernels, name), _name=name, **options):
+            called.setdefault(_name, []).append(options.get("beside"))
+            return _call(*args, **options)
+        monkeypatch.setattr(kernels, name, counted)
+    lengths = {"a": 20, "b": 333, "c": 700}
+    ids = {rid: random_ids(n + 20, vocab, n) for rid, n in lengths.items()}
+    prompt = random_ids(300 * 5, vocab, 9)
+
+    def run(core, turns):
+        for rid, n in lengths.items():
+            core.cache.add_request(rid)
+            core.runner.run([StepEntry(rid, ids[rid][:n])])
+        core.cache.add_request("p")
+        logits = []
+        for turn in range(turns):
+            entries = [StepEntry(rid, [ids[rid][n + turn]], [0]) for rid, n in lengths.items()]
+            entries.append(StepEntry("p", prompt[300 * turn:300 * (turn + 1)], [299]))
+            logits.append(core.runner.run(entries).clone())
+        core.runner.check_status()
+        for rid in (*lengths, "p"):
+            core.cache.free_request(rid)
+        return torch.stack(logits)
+
+    want = run(eager, 5)
+    called.clear()
+    got = run(captured, 5)                              # eager, captured, three replays
+    assert len(captured.runner._shape_graphs) == 1 and not eager.runner._shape_graphs
+    if dtype == "float32":
+        assert len(called["gemm_f32_split"]) > 0
+    elif kind == "starcoder2":
+        assert True in called["paged_attention_tc"] and len(called["gemm_columns"]) > 0
+    # the same kernels on the same numbers: bit for bit
+    assert bool(got.isfinite().all()) and torch.equal(got, want)
+    again = run(captured, 5)                            # replays only, on other pages
+    if dtype == "float32":                              # a captured prompt of 20 tokens shares its keys out as for the longest
+        assert float((again - want).abs().max()) <= 2e-5
+    else:
+        assert torch.equal(again, want)
