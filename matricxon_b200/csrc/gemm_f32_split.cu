@@ -1,13 +1,23 @@
-// out[M,N] = epilogue(A[M,K] . W[N,K]^T + bias[N]), all float, on the tensor cores, no less exact than the FP32 cores:
-// products of the 32-bit path.
+// out[M,N] = epilogue(A[M,K] . W[N,K]^T + bias[N]), all float, on the tensor cores: products of the 32-bit path.
 //
-// A float is the sum of three bfloat16 numbers, exactly: x = h + m + l with h = bf16(x), m = bf16(x - h), l = x - h - m
-// (8 + 8 + 8 bits of significand and the signs). Of the nine products of two such sums the six largest are formed,
-// h h, h m, m h, m m, h l, l h; what is left out is below 2^-26 of a term. The tensor cores add in float but cut sums off
+// A float of 2^-110 or more is the sum of three bfloat16 numbers, exactly: x = h + m + l with h = bf16(x), m = bf16(x - h),
+// l = x - h - m (8 + 8 + 8 bits of significand and the signs); of smaller ones what lies below bfloat16's smallest number,
+// 2^-133, is lost. Of the nine products of two such sums the six largest are formed, h h, h m, m h, m m, h l, l h; what is left
+// out is at most 2^-24 of a term (|m| reaches 2^-8 of a float, |l| 2^-17). The tensor cores add in float but cut sums off
 // instead of rounding them, so an accumulator only ever holds 32 values of k, the small products first and h h last; it is
 // then added to float registers, rounded to nearest (96 additions for K = 3,072, where the FP32 cores' chains make 768 to a
-// piece). Root mean square error against 64 bits, of the result's: 1.1e-7 to 1.9e-7 for K = 3,072 (by the shares of K; the FP32
-// cores 5.0e-7), 1.8e-7 to 3.6e-7 for K = 12,288 (1.0e-6).
+// piece).
+// Root mean square error against 64 bits, of the result's, here and on the FP32 cores, K = 512 / 3,072 / 12,288:
+//   operands of both signs        8.1e-8 and 2.1e-7    1.1e-7 and 5.0e-7    1.5e-7 and 9.9e-7
+//   of one sign (|normal|)        6.3e-8 and 8.5e-8    7.2e-8 and 2.1e-7    7.9e-8 and 4.1e-7
+//   relu^2 times |normal|         7.0e-8 and 7.3e-8    7.5e-8 and 1.5e-7    8.2e-8 and 3.1e-7
+//   one term 10,000 x the others  9.3e-8 and 2.1e-7    1.1e-7 and 4.7e-7    1.5e-7 and 9.7e-7
+//   one value in fifty not zero   6.8e-8 and 5.3e-8    8.8e-8 and 8.3e-8    1.2e-7 and 1.5e-7
+//   one value alone               4.5e-8 and 2.6e-8    4.5e-8 and 2.5e-8    4.6e-8 and 2.5e-8
+// So sums of many terms come closer, of one sign too; rows of few terms do not, since the FP32 cores then round little.
+// The order of a row's sums, and the unit that forms them, follow the number of rows: FP32 cores up to two, mma.sync up to
+// eight, tcgen05 above, with shares of K that depend on the tiles. The same row in another batch differs in its last bits, as
+// in bfloat16; gemm_backend "simt" keeps every product on the FP32 cores, where it does not.
 // A result that is not finite (an operand that is not, an overflow on the way, a float above bfloat16's largest) is formed
 // again from the operands by plain multiply-adds, which decide what it is, unless its row of A holds a NaN, which decides it:
 // a warp looks at the row first (one such row among 4 of 3,072 x 12,288 took 558 us as chains and takes 40, the product 40;
