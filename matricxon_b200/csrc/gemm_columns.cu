@@ -8,7 +8,7 @@
 // tokens, so 16 KB + 64 bytes a token for 64 of K), a ring of TMA stages feeds it through its tiles without a break, and two
 // accumulators let the eight epilogue warps of a block store one tile under the next one's products. Where the result is a
 // sum added to the stream in place, K is also shared out: every part leaves its sums in scratch memory, and whoever reads the
-// stream next (the norm, mx_layernorm_sum), or else a kernel of its own, adds them in the order of K, so that a product
+// stream next (the norm: mx_layernorm_sum, mx_rmsnorm_pending), or else a kernel of its own, adds them in order, so a product
 // repeats bit by bit. Product and norm, us, against adding to memory in the order in which the parts end, which does not
 // repeat: 367 x 3,072 x 12,288 35.2 and 33.1, 512 rows 40.6 and 39.3, 1,024 x 1,024 x 6,144 21.2 and 21.2, 2,048 rows 30.0 and
 // 30.7 (35 to 44 with K in one piece); parts that meet in the shared memory of clusters of four or six blocks take 3 to 7 us

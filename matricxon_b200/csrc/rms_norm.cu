@@ -215,11 +215,12 @@ __global__ void rmsnorm_vec_kernel(const float* x, const int* __restrict__ rows,
 }
 
 // The same behind a residual sum that is still to be formed: the row is x + (acc + col_bias), written back on the way (`acc`
-// null: x + col_bias).
+// null: x + col_bias). With `parts` (a product left in parts of K, [n_parts][rows][hidden], `plane` apart, added up in their
+// order) their sum joins x first, or col_bias where there is no acc.
 template <typename TOut>
 __global__ void rmsnorm_pending_vec_kernel(float* x, const float* acc, const float* __restrict__ col_bias,
                                            const float* __restrict__ weight, float offset, TOut* __restrict__ out,
-                                           int hidden, float eps) {
+                                           int hidden, float eps, const float* parts, int n_parts, size_t plane) {
     __shared__ float scratch[32];
     pdl_trigger();
     const int r = blockIdx.x;
@@ -233,14 +234,39 @@ __global__ void rmsnorm_pending_vec_kernel(float* x, const float* acc, const flo
     pdl_wait();
     float4* xr = reinterpret_cast<float4*>(after_wait(x) + (size_t)r * hidden);
     const float4* ar = acc ? reinterpret_cast<const float4*>(after_wait(acc) + (size_t)r * hidden) : nullptr;
-    float4 kept[RMS_VEC];
+    float4 kept[RMS_VEC], sum[RMS_VEC];                       // sum: of the parts
+    if (n_parts > 0) {
+        const float* pr = after_wait(parts) + (size_t)r * hidden;
+#pragma unroll
+        for (int n = 0; n < RMS_VEC; ++n) {
+            const int i = threadIdx.x + n * blockDim.x;
+            if (i < vecs) sum[n] = reinterpret_cast<const float4*>(pr)[i];
+        }
+        for (int p = 1; p < n_parts; ++p) {
+            float4 more[RMS_VEC];
+#pragma unroll
+            for (int n = 0; n < RMS_VEC; ++n) {
+                const int i = threadIdx.x + n * blockDim.x;
+                if (i < vecs) more[n] = reinterpret_cast<const float4*>(pr + p * plane)[i];
+            }
+#pragma unroll
+            for (int n = 0; n < RMS_VEC; ++n) {
+                if (threadIdx.x + n * blockDim.x >= vecs) continue;
+                sum[n].x += more[n].x; sum[n].y += more[n].y; sum[n].z += more[n].z; sum[n].w += more[n].w;
+            }
+        }
+    }
     float s = 0.f;
 #pragma unroll
     for (int n = 0; n < RMS_VEC; ++n) {
         const int i = threadIdx.x + n * blockDim.x;
         if (i < vecs) {
-            const float4 a = xr[i];
+            float4 a = xr[i];
             float4 b = ar ? ar[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (n_parts > 0) {
+                if (ar) { a.x += sum[n].x; a.y += sum[n].y; a.z += sum[n].z; a.w += sum[n].w; }
+                else b = sum[n];
+            }
             if (col_bias) {
                 const float4 c = reinterpret_cast<const float4*>(col_bias)[i];
                 b.x += c.x; b.y += c.y; b.z += c.z; b.w += c.w;
@@ -381,25 +407,34 @@ extern "C" int mx_add_row(float* x, const float* vector, int n_rows, int hidden,
     return mx_launch_status();
 }
 
-extern "C" int mx_rmsnorm_pending(float* x, const float* acc, const float* col_bias, const float* weight, float offset,
-                                  void* out, int out_dtype, int n_rows, int hidden, float eps, cudaStream_t stream) {
+extern "C" int mx_rmsnorm_pending(float* x, const float* acc, const float* parts, int n_parts, const float* col_bias,
+                                  const float* weight, float offset, void* out, int out_dtype, int n_rows, int hidden, float eps,
+                                  cudaStream_t stream) {
     if (n_rows <= 0) return MX_OK;
     if (hidden <= 0) MX_REFUSE("rmsnorm: hidden must be positive, got %d", hidden);
-    if (acc == nullptr && col_bias == nullptr) MX_REFUSE("rmsnorm of a pending sum: nothing to add");
-    const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(acc) |
+    if (parts == nullptr) n_parts = 0;
+    if (n_parts < 0 || n_parts > MX_SUM_PARTS) MX_REFUSE("rmsnorm of a pending sum: %d parts", n_parts);
+    if (acc == nullptr && n_parts == 0 && col_bias == nullptr) MX_REFUSE("rmsnorm of a pending sum: nothing to add");
+    const size_t plane = (size_t)n_rows * hidden;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(acc) | reinterpret_cast<uintptr_t>(parts) |
                            reinterpret_cast<uintptr_t>(col_bias) | reinterpret_cast<uintptr_t>(weight) |
                            reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     const int vec_threads = aligned ? vec_threads_for(n_rows, hidden) : 0;
     if (vec_threads > 0) {
         if (out_dtype == MX_DTYPE_F32)
             mx_launch_chained(rmsnorm_pending_vec_kernel<float>, dim3(n_rows), dim3(vec_threads), 0, stream, x, acc,
-                              col_bias, weight, offset, (float*)out, hidden, eps);
+                              col_bias, weight, offset, (float*)out, hidden, eps, parts, n_parts, plane);
         else
             mx_launch_chained(rmsnorm_pending_vec_kernel<__nv_bfloat16>, dim3(n_rows), dim3(vec_threads), 0, stream, x,
-                              acc, col_bias, weight, offset, (__nv_bfloat16*)out, hidden, eps);
+                              acc, col_bias, weight, offset, (__nv_bfloat16*)out, hidden, eps, parts, n_parts, plane);
         return mx_launch_status();
     }
     // rows that the float4 kernel does not take: the sum by the epilogue kernel, then the norm
+    if (n_parts > 0) {
+        const int rc = mx_add_parts(parts, hidden, n_parts, acc ? nullptr : col_bias, x, hidden, n_rows, hidden, stream);
+        if (rc != MX_OK) return rc;
+        if (acc == nullptr) return mx_rmsnorm(x, nullptr, weight, offset, out, out_dtype, n_rows, hidden, eps, hidden, stream);
+    }
     const int rc = acc ? mx_epilogue(acc, MX_DTYPE_F32, col_bias, x, x, MX_DTYPE_F32, n_rows, hidden, MX_MODE_RESIDUAL, stream)
                        : mx_add_row(x, col_bias, n_rows, hidden, stream);
     if (rc != MX_OK) return rc;

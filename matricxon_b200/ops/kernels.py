@@ -7,6 +7,8 @@ is an error, not a cue to fall back.
 
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from matricxon_b200.ops.library import KernelLibraryError, check, library
@@ -208,6 +210,7 @@ def split_gemm_supported(a: torch.Tensor, w: torch.Tensor) -> bool:
             and a.stride(0) % 4 == 0 and (a.shape[0] <= 1 or a.stride(0) >= a.shape[1]) and w.is_contiguous() and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+@functools.lru_cache(maxsize=4096)
 def split_gemm_pays(m: int, n: int, k: int) -> bool:
     """Whether a float product that the split kernel takes is better off there than on the FP32 cores
     (gemm_f32_split.cu)."""
@@ -292,6 +295,7 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None,
     _launched()
 
 
+@functools.lru_cache(maxsize=4096)
 def columns_gemm_pays(m: int, n: int, k: int) -> bool:
     """Whether a product of more than 256 rows is better off with its tokens as columns (gemm_columns.cu)."""
     return bool(library().mx_gemm_columns_pays(m, n, k))
@@ -325,6 +329,7 @@ def gemm_columns(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None,
     _launched(2 if n_parts > 1 else 1)
 
 
+@functools.lru_cache(maxsize=4096)
 def columns_gemm_parts(m: int, n: int, k: int) -> int:
     """Parts of K that ``gemm_columns`` cuts a product into that is added to the stream in place (1: none)."""
     return library().mx_gemm_columns_parts(m, n, k)
@@ -340,7 +345,7 @@ def gemm_columns_in_parts(a: torch.Tensor, w: torch.Tensor, residual: torch.Tens
     n = w.shape[0]
     n_parts = columns_gemm_parts(m, n, k)
     assert w.shape[1] == k and tuple(residual.shape) == (m, n) and n % 4 == 0 and n_parts > 1, (a.shape, w.shape, n_parts)
-    parts = torch.empty((n_parts, m, n), dtype=torch.float32, device=a.device)
+    parts = residual.new_empty((n_parts, m, n))
     check(library().mx_gemm_columns(_ptr(a), _ptr(w), None, _ptr(residual), _ptr(residual), dtype_code(torch.float32),
                                     _ptr(parts), 0, m, n, k, a.stride(0), w.stride(0), residual.stride(0), EPILOGUE_RESIDUAL,
                                     _ptr(default_status(a.device)), _stream()), "gemm_columns")
@@ -708,10 +713,11 @@ def add_row(x: torch.Tensor, vector: torch.Tensor) -> None:
 
 
 def rmsnorm_pending(x: torch.Tensor, acc: torch.Tensor | None, col_bias: torch.Tensor | None, weight: torch.Tensor,
-                    offset: float, eps: float, out: torch.Tensor) -> None:
+                    offset: float, eps: float, out: torch.Tensor, parts: torch.Tensor | None = None) -> None:
     """``x += acc + col_bias`` (the residual epilogue of a product whose float accumulator is ``acc``; None: the vector
     alone), then
-    ``out = x / sqrt(mean(x^2) + eps) * (offset + weight)``, in one pass over the rows."""
+    ``out = x / sqrt(mean(x^2) + eps) * (offset + weight)``, in one pass over the rows. ``parts`` [parts, rows, columns]: a
+    product left in parts of K is added too, before ``acc``."""
     _need(x, "x", torch.float32)
     if acc is not None:
         _need(acc, "acc", torch.float32)
@@ -722,8 +728,11 @@ def rmsnorm_pending(x: torch.Tensor, acc: torch.Tensor | None, col_bias: torch.T
     if col_bias is not None:
         _need(col_bias, "col_bias", torch.float32)
         assert col_bias.numel() == x.shape[1]
-    check(library().mx_rmsnorm_pending(_ptr(x), _ptr(acc), _ptr(col_bias), _ptr(weight), float(offset), _ptr(out),
-                                       dtype_code(out.dtype), x.shape[0], x.shape[1], float(eps), _stream()),
+    if parts is not None:
+        _need(parts, "parts", torch.float32)
+        assert parts.shape[1:] == x.shape
+    check(library().mx_rmsnorm_pending(_ptr(x), _ptr(acc), _ptr(parts), 0 if parts is None else parts.shape[0], _ptr(col_bias),
+                                       _ptr(weight), float(offset), _ptr(out), dtype_code(out.dtype), x.shape[0], x.shape[1], float(eps), _stream()),
           "rmsnorm_pending")
     _launched()
 

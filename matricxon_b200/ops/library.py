@@ -58,7 +58,7 @@ _SIGNATURES: dict[str, tuple[list, object]] = {
     "mx_paged_attention": ([P, I, I, P, L, I, P, I, P, P, I, I, I, I, I, F, P, I, I, P, P, F, P, I, P, P], I),
     "mx_rmsnorm": ([P, P, P, F, P, I, I, I, F, L, P], I),
     "mx_add_row": ([P, P, I, I, P], I),
-    "mx_rmsnorm_pending": ([P, P, P, P, F, P, I, I, I, F, P], I),
+    "mx_rmsnorm_pending": ([P, P, P, I, P, P, F, P, I, I, I, F, P], I),
     "mx_rmsnorm_branch_add": ([P, P, P, P, P, I, I, I, F, P], I),
     "mx_rmsnorm_sum": ([P, P, F, P, F, P, I, I, I, F, P], I),
     "mx_cast_rows": ([P, P, L, P], I),

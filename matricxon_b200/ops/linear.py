@@ -1,21 +1,24 @@
 """``out = epilogue(x @ W.T + bias)``: the one matrix product every part uses.
 
 Backends, chosen by the runtime:
-  "simt"    -- the engine's own FP32-core kernels.
-  "split"   -- the engine's tcgen05 kernel of the 32-bit path: each float as three bfloat16 numbers.
+  "simt"    -- the engine's own FP32-core kernels. On the 32-bit path they alone give a row the same bits whatever
+               the number of rows.
+  "split"   -- the engine's tensor-core kernels of the 32-bit path: each float as three bfloat16 numbers ("auto" only).
   "skinny"  -- the engine's tensor-core kernel for at most 16 rows (decoding): the weight
                matrix is streamed once and the epilogue is fused.
   "stream"  -- the engine's TMA + tcgen05 kernel for at most 128 rows with the tokens as the
                narrow side of the product: one block per SM streams its share of the weight rows.
   "tcgen05" -- the engine's TMA + tcgen05 kernels for prompt-sized products with tiles of 128, 256 or 512
-               tokens: operands staged by TMA, accumulator in tensor memory, epilogue fused.
+               tokens: operands staged by TMA, accumulator in tensor memory, epilogue fused. "auto" takes the 512-row
+               kernel alone; the 256-row one, on request, adds parts of K in no fixed order.
   "columns" -- the same with the tokens as the columns of pairs of SMs, in tiles of any multiple of 16.
   "library" -- cuBLAS through ``torch.mm`` for bfloat16 (the reference runs its products
                through nn.Linear, i.e. the library: app/architectures/qwen_layers.py:50-53),
                followed by the engine's fused bias / GELU / residual epilogue kernel.
-  "auto"    -- for float32 "split" where it pays, else "simt"; for bfloat16 "skinny" up to 16 rows, "columns" or "tcgen05" above 256 rows,
-               "library" between (a weight stream that 128-row tiles would leave to a few SMs) and
-               for shapes neither takes (a K that is no multiple of 8), and "stream" from 9 rows
+  "auto"    -- for float32 "split" where it pays, else "simt"; for bfloat16 "skinny" up to 16 rows, "columns" or,
+               from 2,048 rows on, "tcgen05" above 256 rows, "library" between (a weight stream that
+               128-row tiles would leave to a few SMs), for projections short in N and K up to 1,023 rows
+               and for shapes neither takes (a K that is no multiple of 8), and "stream" from 9 rows
                on for large matrices (``_pick`` gives the measured thresholds).
 """
 
@@ -79,13 +82,12 @@ def _pick(x: torch.Tensor, weight: torch.Tensor, m: int, n: int) -> str:
             return "stream"
     if kernels.skinny_gemm_supported(x, weight):
         return "skinny"
-    # up to 256 rows a product has one row of 256-row tiles and too few of them for 148 SMs (each is
-    # bound by what one SM takes in through TMA): the library is faster there (73 against 86 us for
-    # the four products of a layer at 256 rows; 104 against 114 at 512, where the long-K product
-    # already favours the engine's kernel)
-    # ... and up to 1,023 rows for products that are short in both N and K (the QKV and output
-    # projections: 14 against 23 and 14 against 18 us at 512 rows), which have too few tiles to fill
-    # the GPU and too little K to share out
+    # up to 256 rows a product has too few tiles for 148 SMs (each is bound by what one SM takes in through TMA):
+    # the library is faster there (73 us for the four products of a layer at 256 rows, 86 with 256-row tiles)
+    # ... and up to 1,023 rows for products that are short in both N and K (the QKV and output projections). Us there
+    # and here: 512 x 3,584 x 3,072 13.7 and 15.8, 512 x 3,072 x 3,072 with the norm that adds it 19.0 and 19.6; but
+    # 1,023 rows 26.7 and 24.5, 512 x 4,608 x 4,608 28.2 and 26.0, 512 x 6,144 x 6,144 48.3 and 41.6: a line drawn
+    # against earlier kernels, which leaves wide output projections to take
     if m > 256 and kernels.tcgen05_gemm_supported(x, weight) and (m >= 1024 or n >= 8192 or x.shape[1] >= 8192):
         return "columns" if kernels.columns_gemm_pays(m, n, x.shape[1]) else "tcgen05"
     return "library"
@@ -96,7 +98,8 @@ class PendingSum:
     more rows, or the parts of K of a "columns" product, handed to the norm that follows, which forms the
     sum on its way through the rows (``kernels.layernorm_sum``) instead of an epilogue pass of its own.
     ``tensor()`` adds it up for anybody else. ``acc`` None: only a vector (``bias``) is still to be added to
-    every row; ``parts`` [parts, rows, columns] (or None): ``acc`` is their sum."""
+    every row; ``parts`` [parts, rows, columns] (or None): ``acc`` is their sum, or, beside an ``acc`` given,
+    those of an earlier product of the same stream (without a bias), which is added first."""
 
     def __init__(self, acc: torch.Tensor | None, bias: torch.Tensor | None, residual: torch.Tensor,
                  parts: torch.Tensor | None = None) -> None:
@@ -106,11 +109,28 @@ class PendingSum:
 
     @property
     def acc(self) -> torch.Tensor | None:
-        """The product as one tensor (formed now if it was left in parts)."""
+        """What is still to be added, without ``bias``, as one tensor (formed now if it was left in parts)."""
         if self.parts is not None:
-            kernels.add_parts(self.parts[1:], None, self.parts[0])
-            self._acc, self.parts = self.parts[0], None
+            if self._acc is None:
+                kernels.add_parts(self.parts[1:], None, self.parts[0])
+                self._acc = self.parts[0]
+            else:
+                kernels.add_parts(self.parts, None, self._acc)
+            self.parts = None
         return self._acc
+
+    @property
+    def acc_apart(self) -> torch.Tensor | None:
+        """``acc`` for a kernel that takes ``parts`` too."""
+        return self._acc
+
+    def and_bias(self, bias: torch.Tensor) -> "PendingSum":
+        """The same with a vector where there is none yet."""
+        return PendingSum(self._acc, bias, self.residual, self.parts)
+
+    def and_earlier(self, parts: torch.Tensor) -> "PendingSum":
+        """The same (not in parts itself) with an earlier product of the stream that was left in ``parts``."""
+        return PendingSum(self._acc, self.bias, self.residual, parts)
 
     @property
     def shape(self):
@@ -131,12 +151,14 @@ class PendingSum:
 
     def tensor(self) -> torch.Tensor:
         if not self._done and self.parts is not None:
-            kernels.add_parts(self.parts, self.bias, self.residual)
-            self._done = True
-        elif not self._done and self.acc is None:
+            alone = self._acc is None
+            kernels.add_parts(self.parts, self.bias if alone else None, self.residual)
+            self._done, self.parts = alone, None
+        if not self._done and self._acc is None:
             kernels.add_row(self.residual, self.bias)
+            self._done = True
         elif not self._done:
-            kernels.epilogue(self.acc, self.bias, self.residual, self.residual, EPILOGUE_RESIDUAL)
+            kernels.epilogue(self._acc, self.bias, self.residual, self.residual, EPILOGUE_RESIDUAL)
             self._done = True
         return self.residual
 

@@ -129,13 +129,26 @@ class PreNormParallelBlock(Block):
 
     def forward(self, x, ctx, binding):
         x, h = PreNormSequentialBlock._normed(self.mixer_norm, x)
-        if self.feed_forward is not None:
-            x = self.feed_forward.forward(h, x, ctx)
+        earlier = None                                  # the feed-forward's product, where it was left in parts of K
         ctx.sums_may_pend = True
         try:
+            if self.feed_forward is not None:
+                x = self.feed_forward.forward(h, x, ctx)
+                if isinstance(x, PendingSum):
+                    if x.parts is not None and x.acc_apart is None and x.bias is None:
+                        earlier, x = x, x.residual
+                    else:
+                        x = x.tensor()
             x = self.mixer.forward(h, x, ctx, binding)
         finally:
             ctx.sums_may_pend = False
+        if earlier is not None:
+            if isinstance(x, PendingSum) and x.parts is None:
+                x = x.and_earlier(earlier.parts)
+            elif isinstance(x, PendingSum):             # both products in parts
+                earlier.tensor()
+            else:                                       # the mixer has added to the stream itself
+                x = earlier
         if isinstance(x, PendingSum) and not getattr(ctx, "pending_sum_wanted", False):
             return x.tensor()
         return x

@@ -43,7 +43,7 @@ class LayerNorm(Norm):
         kernel forms the sum, writes it to the residual stream and normalises it. Returns (x, norm(x))."""
         x = pending.added_by_kernel()
         out = torch.empty(tuple(x.shape), dtype=self.runtime.dtype, device=x.device)
-        acc = pending.parts if pending.parts is not None else pending.acc
+        acc = pending.parts if pending.parts is not None and pending.acc_apart is None else pending.acc
         kernels.layernorm_sum(x, acc, pending.bias, self.weight, self.bias, self.spec.eps, out)
         return x, out
 
@@ -96,7 +96,7 @@ class RmsNorm(Norm):
         kernel. Returns (x, norm(x))."""
         x = pending.added_by_kernel()
         out = torch.empty(tuple(x.shape), dtype=self.runtime.dtype, device=x.device)
-        kernels.rmsnorm_pending(x, pending.acc, pending.bias, self.weight, self.offset, self.spec.eps, out)
+        kernels.rmsnorm_pending(x, pending.acc_apart, pending.bias, self.weight, self.offset, self.spec.eps, out, pending.parts)
         return x, out
 
     def forward_scaled_sum(self, x, sublayer, skip_scale):

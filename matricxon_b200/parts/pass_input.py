@@ -96,6 +96,6 @@ class StepVector(PassInput):
         step = self.steps[pass_index]
         if isinstance(x, PendingSum):
             if x.bias is None:
-                return PendingSum(x.acc, step, x.residual)
+                return x.and_bias(step)
             x = x.tensor()
         return PendingSum(None, step, x)

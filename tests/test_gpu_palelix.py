@@ -719,3 +719,56 @@ def test_trace_program_and_command_line(tmp_path):
                           timeout=600, cwd=str(ROOT))
     assert done.returncode == 0, done.stderr[-2000:]
     assert "finish_reason:  length" in done.stdout and "Palelix" in done.stdout
+
+
+@pytest.mark.parametrize("rows,hidden", [(9, 2048), (300, 1000), (5, 1002), (3, 24576)])
+def test_parts_of_a_product_join_what_is_still_to_be_added(rows, hidden):
+    """A product left in parts of K, alone or before another one's float result: the norm, and whoever asks for the stream or
+    for one tensor, add the same."""
+    gen = torch.Generator().manual_seed(hidden)
+    x, acc = (torch.randn(rows, hidden, generator=gen).to(DEVICE) for _ in range(2))
+    vector, weight = (torch.randn(hidden, generator=gen).to(DEVICE) for _ in range(2))
+    parts = torch.randn(3, rows, hidden, generator=gen).to(DEVICE)
+    product = (parts[0] + parts[1]) + parts[2]
+    for bias in (None, vector):
+        added = 0.0 if bias is None else bias
+        for there, want in ((None, x + (product + added)), (acc, (x + product) + (acc + added))):
+            def pending():
+                return PendingSum(None if there is None else there.clone(), bias, x.clone(), parts.clone())
+
+            stream, out, alone = x.clone(), torch.empty(rows, hidden, device=DEVICE), torch.empty(rows, hidden, device=DEVICE)
+            kernels.rmsnorm_pending(stream, there, bias, weight, 0.0, 1e-4, out, parts)
+            kernels.rmsnorm(want, weight, 0.0, 1e-4, alone)
+            # a sum of five terms in another order
+            close = lambda one, two: bool(((one - two).abs() <= 6 * 2.0 ** -23 * (x.abs() + parts.abs().sum(0) + acc.abs() + vector.abs())).all())
+            assert close(stream, want) and torch.allclose(out, alone, rtol=1e-5, atol=1e-5)
+            asked = pending()
+            assert close(asked.tensor(), want) and torch.equal(asked.tensor(), asked.residual)
+            asked = pending()
+            assert close(asked.acc, product + (0.0 if there is None else there)) and asked.parts is None
+            assert close(asked.tensor(), want)
+    both = PendingSum(acc.clone(), None, x.clone()).and_earlier(parts).and_bias(vector)
+    assert bool(((both.tensor() - ((x + product) + (acc + vector))).abs() <= 1e-4).all())
+
+
+def test_a_feed_forward_in_parts_waits_for_the_next_norm():
+    """Mixer and feed-forward on one norm, 300 rows of a width whose down product is cut into parts of K: two layers whose sums
+    wait for the next norm give what they give when every layer adds up its own."""
+    from matricxon_b200.ops import kernels as k
+    from palelix_configs import config_of, dense, lightning, model
+
+    raw = model(1024, 200, [lightning(4, 64, 64, [0.9, 0.97, 0.99, 0.998], mlp=dense(8192)) for _ in range(3)])
+    assert k.columns_gemm_parts(300, 1024, 8192) > 1
+    from matricxon_b200.engine.step import StepEntry
+
+    tokens, logits = ids(300, 200, seed=9), []
+    for taps in (False, True):                          # a caller that wants every layer's stream has it added up there
+        core = Run(raw, draw(raw, seed=4), "bfloat16", max_tokens=512, max_requests=1).replayer.core
+        if taps:
+            core.runner.taps = ("layer_outputs",)
+        core.cache.add_request("r")
+        logits.append(core.runner.run([StepEntry("r", tokens, [299])]).clone())
+        core.runner.check_status()
+    size = float(logits[1].abs().max())
+    # one rounding to bfloat16 a layer may fall the other way
+    assert float((logits[0] - logits[1]).abs().max()) <= 3 * 2.0 ** -7 * size
