@@ -317,7 +317,9 @@ paged_attention_kernel(const AttnParams p) {
 // with a softmax of its own, and are combined at the end. Up to six heads a block, so that four blocks fit an SM: eight warps
 // of twelve heads hide too little (a prompt of 389 tokens, 24 heads on 2: 126 us, 100 with six; 200 tokens, 16 on 2: 39 and
 // 30), though keys and values are then read twice. Bound by the multiply-adds of long prompts (two thirds of the
-// instructions) and by one trip to memory in decoding. Steps of eight layers at the 3B sizes: a prompt of 389 tokens 5,806 ->
+// instructions) and by one trip to memory in decoding. Against the kernel above over 1, 2 and 8 KV heads with 1 to 24 query heads
+// each (1 to 3 compute four, 7 to 12 read keys and values twice): one request of 700 tokens 7.9 us and 29 (1 on 1), 11.3 and 32
+// (24 on 2), four of 4,096 22.9 and 43.9, 31.7 and 53.2, a prompt of 900 85 and 472, 405 and 819; no shape was slower. Steps of eight layers at the 3B sizes: a prompt of 389 tokens 5,806 ->
 // 5,131 us, four requests of 490 to 701 tokens 1,581 -> 1,397; with six heads a block and the split products for few rows 5,221
 // -> 5,111 and 1,108 -> 1,071.
 constexpr int F32A_KEYS = 16, F32A_DIM = 128;

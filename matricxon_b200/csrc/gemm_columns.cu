@@ -312,9 +312,10 @@ double cl_plan(int M, int N, int K, bool may_split, int pairs, ClPlan* best) {
 // Whether a product of more than 256 rows that fills the SMs is better off here than on the kernels with 128, 256 or 512
 // tokens to a tile (gemm_tcgen05.cu). Us there against here, weights from HBM: with GELU 367 x 12,288 x 3,072 36.1 and 27.8,
 // 512 38.9 and 33.2, 543 x 18,432 x 4,608 104 and 72, 1,023 x 12,288 x 3,072 75.7 and 60.0, 1,777 x 16,384 x 2,048 106 and 88;
-// added to the stream 367 x 3,072 x 12,288 37.4 and 27.4, 512 35.0 and 33.5, 543 x 4,608 x 18,432 94.7 and 73.0, 1,400 x 3,072
-// x 3,072 30.6 and 26.1, 2,048 x 2,048 x 8,192 65 and 56; 8,192 x 12,288 x 3,072 459 and 385 (GELU). From 2,048 rows on
-// 512-row tiles are as good where K is long and the result narrow: 2,048 x 4,608 x 18,432 221 and 232, 2,500 x 3,072 x 12,288
+// 8,192 x 12,288 x 3,072 459 and 385; added to the stream, with the norm that reads it, 367 x 3,072 x 12,288 43.7 and 34.8, 512
+// 42.0 and 40.6, 633 x 2,048 x 8,192 37.5 and 29.4, 543 x 4,608 x 18,432 99 and 72, 1,024 x 1,024 x 6,144 26.3 and 21.2, 1,400 x
+// 3,072 x 3,072 39.9 and 32.4, 2,048 x 1,024 x 6,144 54.6 and 30.0 (in two parts of K; in one 35), 2,048 x 2,048 x 8,192 76 and
+// 57. From 2,048 rows on 512-row tiles are as good where K is long and the result narrow: 2,048 x 4,608 x 18,432 221 and 232, 2,500 x 3,072 x 12,288
 // 127 and 134, 4,096 x 2,048 x 8,192 96 and 100, 8,192 x 1,024 x 6,144 75 and 84.
 extern "C" int mx_gemm_columns_pays(int M, int N, int K) {
     return M > 256 && !(M >= 2048 && N < K && K >= (M >= 8192 ? 6144 : M >= 4096 ? 8192 : 12288));

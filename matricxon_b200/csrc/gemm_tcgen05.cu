@@ -25,8 +25,11 @@
 // the status word and the role moves on, so the block always reaches the point where tensor
 // memory is freed.
 //
-// Three kernels share this scheme: 128-row tiles (below), 256-row tiles (two accumulators per block) and
-// 512-row tiles on pairs of SMs (cta_group::2); mx_gemm_tcgen05 picks by the number of rows.
+// Three kernels share this scheme: 128-row tiles (below; also the grouped product of the experts), 256-row tiles
+// (two accumulators per block) and 512-row tiles on pairs of SMs (cta_group::2). mx_gemm_tcgen05 picks by the number
+// of rows. Where the engine chooses for itself it comes here with 2,048 rows and more only (gemm_columns.cu takes the
+// rest), and so to the 512-row kernel, or to the 128-row one for results that are not aligned; the 256-row kernel and
+// the choice below 2,048 rows are for callers that ask for gemm_backend "tcgen05".
 //
 // Epilogue modes as in gemm_simt.cu: 0 out(bf16) = v; 1 out(bf16) = gelu_tanh(v);
 // 2 out(f32) = residual + v; 3 out(f32) = v; 4 out(bf16) = max(v, 0)^2, with v = acc + bias.
@@ -1057,6 +1060,7 @@ extern "C" int mx_gemm_tcgen05(const void* A, const void* W, const float* bias, 
                            (bias == nullptr || reinterpret_cast<uintptr_t>(bias) % 16 == 0);
     // a residual added in place lets K be shared out between blocks (every part adds into the output)
     const bool may_split = mode == 2 && residual == out && vector_ok && split_k_allowed();
+    // (below 2,048 rows on explicit request only: see the top)
     // 512-row tiles on pairs of SMs from 2,048 rows on (below that its tiles are too few or too narrow: at
     // 1,024 rows the other two are a quarter faster); 256-row tiles (two accumulators per W
     // tile) from 257 rows on, or from 129 when K can be split, unless 128-row tiles give every SM four or

@@ -501,8 +501,9 @@ class StepRunner:
             n_tokens = sum(len(entry.tokens) for entry in entries)
             buffers = self._graph_buffers(n_tokens, len(entries), widths)
             ctx = self.build(entries, table_widths=widths, buffers=buffers)
-            # (kernels start while their predecessor drains, as in the decode graphs: a portion of 512 tokens beside 31
-            # requests at the 7B sizes 2,538 -> 2,517 us, a prompt of 1,391 in portions at the 3B sizes 11,757 -> 11,640)
+            # (kernels start while their predecessor drains, as in the decode graphs, here alone: a shape that is new runs
+            # eagerly, kernel after kernel. A portion of 512 tokens beside 31 requests at the 7B sizes 2,538 -> 2,517 us, a
+            # prompt of 1,391 in portions at the 3B sizes 11,757 -> 11,640)
             # a memory pool apart from the decode graphs': their small buffers then stay close together
             # instead of being scattered through the blocks that prompt-sized steps leave behind
             graph, static_logits, launches = self._capture(ctx, False, n_tokens <= self.chained_launch_rows, "_shape_pool")

@@ -71,7 +71,7 @@ class Runtime:
     device: torch.device
     dtype: torch.dtype                    # activations, matrices and cache: bfloat16 or float32
     page_size: int = 16
-    gemm_backend: str = "auto"            # "auto" | "simt" | "library" | "tcgen05"
+    gemm_backend: str = "auto"            # one of ops/linear.py's backends; float32: "auto" or "simt"
 
     def __post_init__(self) -> None:
         self.device = torch.device(self.device)
