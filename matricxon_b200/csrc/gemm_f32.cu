@@ -337,6 +337,7 @@ int mx_gemm_f32(const float* A, int lda, const float* W, int ldw, const float* b
         const dim3 grid(F32_PIECES * ((M + FT_M - 1) / FT_M), (N + FT_N - 1) / FT_N);
         gemm_f32_tile_kernel<<<grid, FT_THREADS, 0, stream>>>(A, lda, W, ldw, bias, residual, out, ldo, M, N, K,
                                                               f32_piece(K), mode);
+        mx_count_launch();
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
